@@ -15,6 +15,7 @@
 // cleared between calls and each point is rebuilt at most once per call.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -60,6 +61,13 @@ constexpr int FLIP_BATCH = 4;       // flip rounds launched before each host che
 // a wave of them, while each further flip round costs its own launches (measured on 4M
 // points, sigma 0.02: repair 1.64 -> 1.49 ms against flipping to the end)
 constexpr int SPILL_EDGES_PER_SM = 64;
+// Work lists of at most this many points per SM go to the warp-per-point kernel whole (two
+// points per resident warp)
+constexpr int WARP_ITEMS_PER_SM = 16;
+// Up to this many points a warp per point throughout: 10,000 points build in 54 us, with a thread
+// per point first in 69 + 66 + 28 us; 45,000 points of a rebuild round in 342 us against 160 + 50 us
+constexpr int WRAP_BUILD_MAX = 20000;
+constexpr int WRAP_REPAIR_MAX = 20000;
 constexpr int MAX_DEFER_CHUNKS = 8;   // slot chunks of an overlapped global build (dgt_set_deferred_overlap)
 constexpr int MAX_FLIP_ROUNDS = 24; // flip rounds of a checked call before the rest is rebuilt
 constexpr int ASYNC_FLIP_ROUNDS = 3; // default flip rounds of an unsynchronised call (best of 1-10 for MD steps at sigma 0.01)
@@ -108,7 +116,7 @@ struct dgt_context {
     int defer_chunks = 1;
     cudaStream_t aux[MAX_DEFER_CHUNKS] = {};
     cudaEvent_t fork_ev = nullptr, aux_ev[MAX_DEFER_CHUNKS] = {};
-    DevBuf dcount;   // deferred count of each piece
+    DevBuf dcount;   // per piece: deferred points, points the first stage handed on, its second pass
 };
 
 namespace {
@@ -137,9 +145,20 @@ struct PhaseTimer {
             c->ev_used[ph] = true;
         }
     }
-    ~PhaseTimer()
+    ~PhaseTimer() { end(); }
+    void end()
     {
         if (c->timing) cudaEventRecord(c->ev[ph][1], s);
+    }
+    // ends this phase and begins the next
+    void next(int p)
+    {
+        end();
+        ph = p;
+        if (c->timing) {
+            cudaEventRecord(c->ev[ph][0], s);
+            c->ev_used[ph] = true;
+        }
     }
 };
 
@@ -234,6 +253,8 @@ void plan_general_set(SetDesc &S, const double m[4], double a, int ns)
     S.icw = xs / S.Lx;
     S.ich = ys / S.Ly;
     S.V = (float)pow2_at_least(std::max(S.Lx, S.Ly));
+    S.per_cell = (float)(ns / ((double)xs * ys));
+    S.star_win = star_window(S.per_cell);
 }
 
 // cell grid of every set from the requested cell edge
@@ -288,6 +309,8 @@ int plan_grid(dgt_context *c)
         S.point_base = pbase;
         S.n = ns;
         S.V = (float)pow2_at_least(std::max(Lx, Ly));
+        S.per_cell = (float)(ns / ((double)xs * ys));
+    S.star_win = star_window(S.per_cell);
         blocks += set_block_grid(S, (int)blocks);
         cells += (long long)xs * ys;
         pbase += ns;
@@ -431,6 +454,17 @@ RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int str
     a.mark = c->mark.as<int>();
     a.defer_list = c->defer_list.as<int>();
     a.defer_count = &c->st.as<DevStatus>()->defer_count;
+    a.star_list = c->rank.as<int>();   // (the binning is done with it)
+    a.star_count = &c->st.as<DevStatus>()->star_count;
+    // a global build has no flips and no repair rounds: their lists hold the first stage's
+    // uncertified points (half of all at most; a sixth of a uniform set)
+    a.second_list = c->list1.as<int>();
+    a.second_count = &c->st.as<DevStatus>()->second_count;
+    a.second_rings[0] = c->flip0.as<int>();
+    a.second_rings[1] = c->flip1.as<int>();
+    a.second_split = c->n / 4;   // 64-byte rings in 16 bytes a point
+    a.second_cap = 2 * a.second_split;
+    a.second_base = 0;
     a.skin = &c->st.as<DevStatus>()->skin;
     a.work_budget = c->work_budget;
     a.check = c->check;
@@ -439,22 +473,32 @@ RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int str
     return a;
 }
 
-// the deferred points (a warp each: long rings, undecided predicates, long scans)
-cudaError_t run_deferred(dgt_context *c, const RingArgs &a, cudaStream_t s)
+// The rings of `a`'s points.  Large sets of points: the first stage with a thread per point
+// (k_star), then with a warp per point (k_wrap) what that could not finish; up to WRAP_BUILD_MAX
+// (repair: WRAP_REPAIR_MAX) points: k_wrap alone, whose latency is far shorter.  What is left goes
+// to the incremental warp kernel (exactly cocircular candidates, circles past half the box, sets
+// of a few cells).  Work budgets too small for the first stage's scans and the kernel shapes with
+// a group of lanes per point leave every point to the incremental kernels instead; the kernel
+// shape applies to those of global triangulations, the rebuild rounds take the default shape.
+cudaError_t run_rings(dgt_context *c, const RingArgs &a, cudaStream_t s, PhaseTimer *build_timer = nullptr)
 {
-    c->launches += 1;
-    return launch_deferred(a, c->sms, s);
-}
-
-// The kernel shape (and the autotuner's choice of it) applies to global triangulations; the
-// rebuild rounds of a repair take the default shape, which is the fastest for their short,
-// latency-bound work lists (measured: 256-set ensemble MD step 0.99 ms against 1.05 ms with
-// the shape tuned for its build; 4M-point repair 1.07 ms against 1.14 ms with shape 1)
-cudaError_t run_build(dgt_context *c, const RingArgs &a, cudaStream_t s)
-{
-    c->launches += a.n_items > 0 ? 1 : 0;
-    return launch_build(a, c->precision == DGT_PRECISION_FP64 ? MODE_F64 : MODE_F32, c->sms,
-                        a.repair ? 0 : c->shape, s);
+    const int mode = c->precision == DGT_PRECISION_FP64 ? MODE_F64 : MODE_F32;
+    const int shape = a.repair ? 0 : c->shape;
+    const int any = a.n_items > 0 ? 1 : 0;
+    cudaError_t e = cudaSuccess;
+    RingArgs b = a;
+    c->launches += any + 1;
+    if (c->work_budget >= STAR_MIN_BUDGET && kernel_shape_lanes(shape) == 1) {
+        b.wrap_items = WRAP_REPAIR_MAX;
+        b.wrap_mode = a.repair ? WRAP_REPAIR : (a.n_items <= WRAP_BUILD_MAX ? WRAP_OWN : WRAP_HANDED);
+        if (b.wrap_mode != WRAP_OWN && (e = launch_star(b, mode, c->sms, &c->launches, s)) != cudaSuccess) return e;
+        if ((e = launch_wrap(b, mode, c->sms, s)) != cudaSuccess) return e;
+        b.worklist = nullptr;
+    } else {
+        if ((e = launch_build(b, mode, c->sms, shape, s)) != cudaSuccess) return e;
+    }
+    if (build_timer) build_timer->next(DGT_PHASE_SLOW);
+    return launch_deferred(b, c->sms, s);
 }
 
 // A global build in c->defer_chunks pieces of the cell order, each on a stream of its own
@@ -467,7 +511,7 @@ cudaError_t run_build(dgt_context *c, const RingArgs &a, cudaStream_t s)
 cudaError_t run_build_chunked(dgt_context *c, const RingArgs &a, cudaStream_t s)
 {
     const int K = c->defer_chunks;
-    cudaError_t e = c->dcount.ensure(sizeof(int) * MAX_DEFER_CHUNKS);
+    cudaError_t e = c->dcount.ensure(sizeof(int) * 3 * MAX_DEFER_CHUNKS);
     if (e != cudaSuccess) return e;
     if (!c->fork_ev && (e = cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming)) != cudaSuccess) return e;
     for (int k = 0; k < K; ++k) {
@@ -476,7 +520,7 @@ cudaError_t run_build_chunked(dgt_context *c, const RingArgs &a, cudaStream_t s)
             return e;
     }
     int *cnt = c->dcount.as<int>();
-    if ((e = cudaMemsetAsync(cnt, 0, sizeof(int) * MAX_DEFER_CHUNKS, s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(cnt, 0, sizeof(int) * 3 * MAX_DEFER_CHUNKS, s)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(c->fork_ev, s)) != cudaSuccess) return e;
     const int per = (c->n + K - 1) / K;
     int used = 0;
@@ -489,8 +533,13 @@ cudaError_t run_build_chunked(dgt_context *c, const RingArgs &a, cudaStream_t s)
         ak.n_items = items;
         ak.defer_list = a.defer_list + lo;
         ak.defer_count = cnt + k;
-        if ((e = run_build(c, ak, c->aux[k])) != cudaSuccess) return e;
-        if ((e = run_deferred(c, ak, c->aux[k])) != cudaSuccess) return e;
+        ak.star_list = a.star_list + lo;
+        ak.star_count = cnt + MAX_DEFER_CHUNKS + k;
+        ak.second_list = a.second_list + lo;
+        ak.second_base = lo / 2;
+        ak.second_cap = std::min(a.second_cap, (lo + items) / 2) - ak.second_base;
+        ak.second_count = cnt + 2 * MAX_DEFER_CHUNKS + k;
+        if ((e = run_rings(c, ak, c->aux[k])) != cudaSuccess) return e;
         if ((e = cudaEventRecord(c->aux_ev[k], c->aux[k])) != cudaSuccess) return e;
         used = k + 1;
     }
@@ -711,14 +760,8 @@ int dgt_global_triangulation(dgt_context *c, const double *d_points, int *d_tri,
         PhaseTimer t(c, DGT_PHASE_BUILD, s);
         DGT_TRY(run_build_chunked(c, a, s));
     } else {
-        {
-            PhaseTimer t(c, DGT_PHASE_BUILD, s);
-            DGT_TRY(run_build(c, a, s));
-        }
-        {
-            PhaseTimer t(c, DGT_PHASE_SLOW, s);
-            DGT_TRY(run_deferred(c, a, s));
-        }
+        PhaseTimer t(c, DGT_PHASE_BUILD, s);
+        DGT_TRY(run_rings(c, a, s, &t));
     }
     c->launches += 1;
     DGT_TRY(launch_call_end(c->ctl.as<DevCtl>(), c->st.as<DevStatus>(), 0, s));
@@ -763,6 +806,7 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
     if (!c->binned) DGT_TRY(run_bin(c, d_points, s));
     else if (!fold) DGT_TRY(run_bin_refresh(c, d_points, s));
     int *lists[2] = { c->list0.as<int>(), c->list1.as<int>() };
+    int *list_counts[2] = { &dst->list_count0, &dst->list_count1 };
     TestArgs t;
     t.sets = c->d_sets.as<SetDesc>();
     t.set_of = c->batch ? c->d_set_of.as<int>() : nullptr;
@@ -776,7 +820,7 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
     t.mark = c->mark.as<int>();
     t.epoch_ptr = &ctl->epoch;
     t.list = lists[0];
-    t.list_count = &dst->list_count[0];
+    t.list_count = list_counts[0];
     int2 *flips[2] = { c->flip0.as<int2>(), c->flip1.as<int2>() };
     t.flip_list = c->flip ? flips[0] : nullptr;
     t.flip_count = &dst->flip_count[0];
@@ -805,7 +849,7 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
         f.mark = t.mark;
         f.epoch_ptr = &ctl->epoch;
         f.rebuild_list = lists[0];
-        f.rebuild_count = &dst->list_count[0];
+        f.rebuild_count = list_counts[0];
         f.claim = c->claim.as<unsigned long long>();
         f.stamp_ptr = &ctl->flip_stamp;
         f.quad = c->quad.as<int2>();
@@ -846,7 +890,7 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
     }
     if (c->flip) {
         c->launches += 1;
-        DGT_TRY(launch_expand(lists[0], &dst->list_count[0], c->n, d_tri, d_nn, stride, c->n, c->mark.as<int>(),
+        DGT_TRY(launch_expand(lists[0], list_counts[0], c->n, d_tri, d_nn, stride, c->n, c->mark.as<int>(),
                               &ctl->epoch, c->sms, s));
     }
     int round = 0;
@@ -856,27 +900,27 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
         int batch = fixed_rounds > 0 ? fixed_rounds : (round == 0 ? FIRST_ROUNDS : NEXT_ROUNDS);
         for (int b = 0; b < batch; ++b, ++round) {
             int cur = round & 1, nxt = cur ^ 1;
-            DGT_TRY(cudaMemsetAsync(&dst->list_count[nxt], 0, sizeof(int), s));
-            DGT_TRY(cudaMemsetAsync(&dst->defer_count, 0, sizeof(int), s));
+            // the next list's count and, between the lists, the deferred and handed-on counts
+            static_assert(offsetof(DevStatus, list_count1) == offsetof(DevStatus, list_count0) + 3 * sizeof(int),
+                          "counters of a round are adjacent");
+            DGT_TRY(cudaMemsetAsync(nxt ? &dst->defer_count : &dst->list_count0, 0, 3 * sizeof(int), s));
             RingArgs a = ring_args(c, d_points, d_tri, d_nn, stride);
             a.worklist = lists[cur];
-            a.worklist_count = &dst->list_count[cur];
+            a.worklist_count = list_counts[cur];
             a.n_items = c->n;
             a.repair = 1;
+            a.count_round = 1;
             a.cand_by_index = 1;
-            // a round of at most 16 points per SM goes to the warp-per-point kernel whole (two
-            // points per resident warp)
-            a.warp_items = c->sms * 16;
+            a.warp_items = c->sms * WARP_ITEMS_PER_SM;
             a.epoch_ptr = &ctl->epoch;
             a.round = round;
             a.next_list = lists[nxt];
-            a.next_count = &dst->list_count[nxt];
-            DGT_TRY(run_build(c, a, s));
-            DGT_TRY(run_deferred(c, a, s));
+            a.next_count = list_counts[nxt];
+            DGT_TRY(run_rings(c, a, s));
         }
         if (fixed_rounds > 0) break;
         int left = 0;
-        DGT_TRY(cudaMemcpyAsync(&left, &dst->list_count[round & 1], sizeof(int), cudaMemcpyDeviceToHost, s));
+        DGT_TRY(cudaMemcpyAsync(&left, list_counts[round & 1], sizeof(int), cudaMemcpyDeviceToHost, s));
         DGT_TRY(cudaStreamSynchronize(s));
         if (left == 0) break;
         if (round > 256) {

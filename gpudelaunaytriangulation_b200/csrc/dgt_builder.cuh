@@ -731,14 +731,14 @@ __device__ __forceinline__ void enqueue_next(const RingArgs &A, int ebase, int e
     if (atomicMax(&A.mark[j], ep + 1) < ebase) A.next_list[atomicAdd(A.next_count, 1)] = j;
 }
 
+// consistency of a rebuilt ring with the rings it touches (repair): queues what it contradicts
 template <class Ring>
-__device__ void finish(const RingArgs &A, int pid, Ring &R, int m, int &maxr)
+__device__ void finish_repair(const RingArgs &A, int pid, const Ring &R, int m)
 {
-    const int ebase = A.repair ? *A.epoch_ptr + 1 : 0;
+    const int ebase = *A.epoch_ptr + 1;
     const int ep = ebase + A.round;
-    maxr = max(maxr, m);
-    int *row = A.tri + (size_t)pid * A.stride;
-    if (A.repair && m <= RR) {
+    const int *row = A.tri + (size_t)pid * A.stride;
+    if (m <= RR) {
         // consistency of the rebuilt ring with the rings it touches (see enqueue rules in
         // dgt_api.cu: points rebuilt in this call are exact; an untouched point must either
         // list pid with the matching neighbours on both sides or be rebuilt too).  Register
@@ -793,7 +793,7 @@ __device__ void finish(const RingArgs &A, int pid, Ring &R, int m, int &maxr)
             }
             if (!ok) enqueue_next(A, ebase, ep, nb.r[k]);
         }
-    } else if (A.repair) {
+    } else {
         int om = A.nn[pid];
         if (om >= 1 && om <= A.stride) {
             for (int k = 0; k < om; ++k) {
@@ -819,6 +819,14 @@ __device__ void finish(const RingArgs &A, int pid, Ring &R, int m, int &maxr)
             if (!ok) enqueue_next(A, ebase, ep, nb);
         }
     }
+}
+
+// a finished ring, rotated to start at its smallest index, into row pid
+template <class Ring>
+__device__ __forceinline__ void store_ring(const RingArgs &A, int pid, const Ring &R, int m, int &maxr)
+{
+    maxr = max(maxr, m);
+    int *row = A.tri + (size_t)pid * A.stride;
     if (m > A.stride) {
         atomicMax(&A.st->need_stride, m);
         A.nn[pid] = 0;   // row left unwritten: mark the ring invalid
@@ -835,6 +843,13 @@ __device__ void finish(const RingArgs &A, int pid, Ring &R, int m, int &maxr)
         row[k] = R.idx(src);
     }
     A.nn[pid] = m;
+}
+
+template <class Ring>
+__device__ void finish(const RingArgs &A, int pid, Ring &R, int m, int &maxr)
+{
+    if (A.repair) finish_repair(A, pid, R, m);
+    store_ring(A, pid, R, m, maxr);
 }
 
 __device__ __forceinline__ void flush_counters(const RingArgs &A, const Ctr &c, unsigned pts, int maxr)

@@ -342,10 +342,6 @@ __global__ void __launch_bounds__(BLOCK) k_build_grp(RingArgs A)
     int maxr = 0;
     const int n = item_count(A);
     if (A.worklist && n <= A.warp_items) return;   // a short work list: k_build_warp takes it
-    if (A.repair && blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
-        atomicAdd(&A.st->repaired, (unsigned long long)n);
-        atomicMax(&A.st->rounds, A.round + 1);
-    }
     for (int base = blockIdx.x * NG; base < n; base += gridDim.x * NG) {
         const int t = base + grp;
         const bool act = t < n;

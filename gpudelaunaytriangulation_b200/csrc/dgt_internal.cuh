@@ -33,6 +33,8 @@ struct SetDesc {
     int sbxsize;        // occupancy super-blocks per row (SBLOCK_CELLS x SBLOCK_CELLS cells each)
     int sbysize;
     int sblock_base;    // first super-block of the set in the block-count array
+    int star_win;       // cells per axis of the first-stage window (dgt_star.cu)
+    float per_cell;     // mean points per cell
     // General periodic box (periodicBoundaries::setGeneral, periodicBoundaries.h:86-101): a
     // point is M u with u its fractional coordinates, and the cell grid is a grid over u, so
     // a cell is a parallelogram.  Used by the kernels' general-box instantiations only; the
@@ -126,9 +128,13 @@ struct DevStatus {
     int max_ring;               // largest ring produced
     int err_flags;              // DGT_EF_* bits
     int rounds;                 // repair rounds executed (device-side count)
-    int list_count[2];          // repair work lists (ping-pong)
+    // one memset clears the next round's list with the two counters between the lists
+    int list_count0;            // repair work lists (ping-pong)
     int defer_count;            // items queued for the warp-per-point kernel
+    int star_count;             // items the first stage handed to the incremental kernels
+    int list_count1;
     int flip_count[2];          // flip candidate lists (ping-pong)
+    int second_count;           // slots for the first stage's second pass (global builds)
     int pad;
     unsigned long long points;          // ring constructions
     unsigned long long candidates;      // candidates examined
@@ -217,6 +223,7 @@ struct RingArgs {
     // repair bookkeeping: this call's base epoch is *epoch_ptr + 1, round r's items carry
     // mark base + r and queue the next round with base + r + 1
     int repair;        // 1: rebuild listed points and propagate consistency checks
+    int count_round;   // 1: this launch counts the round and its items in the status
     int *mark;
     const int *epoch_ptr;
     int round;
@@ -227,6 +234,19 @@ struct RingArgs {
     // scans longer than work_budget (cells + candidates)
     int *defer_list;
     int *defer_count;
+    // points the first stage (dgt_star.cu) hands to the incremental kernels, complemented when
+    // their scan was too large for it
+    int *star_list;
+    int *star_count;
+    // global builds: slots its first pass could not certify, at most second_cap, and their rings,
+    // 16 words each: entry k is number second_base + k over the two arrays, the first of which holds
+    // second_split.  No room (0): both passes run in one launch
+    int wrap_mode;     // which points k_wrap takes (WRAP_*)
+    int wrap_items;    // repair: lists of at most this many points go to k_wrap whole
+    int *second_list;
+    int *second_count;
+    int *second_rings[2];
+    int second_cap, second_base, second_split;
     int item_base;     // without a work list: item t is slot item_base + t
     int work_budget;
     int warp_items;    // work lists of at most this many items are rebuilt by the warp kernel alone
@@ -331,7 +351,26 @@ cudaError_t launch_gather_points(const double2 *src, const int *order, int n, do
 constexpr int KERNEL_SHAPES = 7;
 int kernel_shape_cap(int shape);
 int kernel_shape_block(int shape);
+int kernel_shape_lanes(int shape);
 cudaError_t launch_build(const RingArgs &a, int mode, int sms, int shape, cudaStream_t s);
+// The first stage of builds and rebuilds with a thread per point (dgt_star.cu); what it cannot
+// finish goes to a.star_list.  It scans at most some 200 cells and candidates a point, so a work
+// budget below STAR_MIN_BUDGET leaves every point to the incremental kernels.  (launches:
+// incremented by the kernels launched)
+constexpr int STAR_MIN_BUDGET = 256;
+cudaError_t launch_star(const RingArgs &a, int mode, int sms, int *launches, cudaStream_t s);
+// The same with a warp per point (dgt_wrap.cu, a.wrap_mode); what it cannot finish goes to the
+// deferred list
+enum : int { WRAP_OWN = 0, WRAP_HANDED = 1, WRAP_REPAIR = 2 };
+cudaError_t launch_wrap(const RingArgs &a, int mode, int sms, cudaStream_t s);
+// window of the first stage: about 26 points of a set with `per_cell` points a cell on average
+// (it takes up to 32), three to nine cells per axis
+inline int star_window(double per_cell)
+{
+    int w = 9;
+    while (w > 3 && (double)w * w * per_cell > 26.0) --w;
+    return w;
+}
 // the one-ring kernel with `lanes` (4 or 8) lanes per point (dgt_group.cu)
 cudaError_t launch_build_group(const RingArgs &a, int mode, int sms, int lanes, cudaStream_t s);
 cudaError_t launch_deferred(const RingArgs &a, int sms, cudaStream_t s);

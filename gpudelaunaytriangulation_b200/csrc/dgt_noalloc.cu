@@ -139,6 +139,8 @@ extern "C" int dgt_global_triangulation_noalloc(const double *d_points, int n, d
     S.point_base = 0;
     S.n = n;
     S.V = (float)pow2_at_least(std::max(Lx, Ly));
+    S.per_cell = (float)(n / ((double)xs * ys));
+    S.star_win = star_window(S.per_cell);
     const int blocks = set_block_grid(S, 0);
     const int cells = xs * ys;
     if ((size_t)blocks > NA_MAX_BLOCKS) return DGT_ERR_INVALID_ARGUMENT;
@@ -201,7 +203,9 @@ extern "C" int dgt_global_triangulation_noalloc(const double *d_points, int n, d
     r.defer_count = &d_st->defer_count;
     r.work_budget = DEFAULT_WORK_BUDGET;
     r.st = d_st;
-    if (launch_build(r, MODE_F32, sms, 0, s) != cudaSuccess) return DGT_ERR_CUDA;
+    // (a warp per point: at most 65,536 of them)
+    r.wrap_mode = WRAP_OWN;
+    if (launch_wrap(r, MODE_F32, sms, s) != cudaSuccess) return DGT_ERR_CUDA;
     if (launch_deferred(r, sms, s) != cudaSuccess) return DGT_ERR_CUDA;
 
     // status into host stack memory (pageable: no pinned buffer is allocated)

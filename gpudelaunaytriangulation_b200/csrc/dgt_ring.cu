@@ -42,11 +42,11 @@ __global__ void __launch_bounds__(BLOCK) k_build(RingArgs A)
     unsigned pts = 0;
     int maxr = 0;
     const int n = item_count(A);
-    if (A.worklist && n <= A.warp_items) return;   // a short work list: k_build_warp takes it
-    if (A.repair && blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
+    if (A.count_round && blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
         atomicAdd(&A.st->repaired, (unsigned long long)n);
         atomicMax(&A.st->rounds, A.round + 1);
     }
+    if (A.worklist && n <= A.warp_items) return;   // a short work list: k_build_warp takes it
     for (int base = blockIdx.x * BLOCK; base < n; base += gridDim.x * BLOCK) {
         // every lane runs the builder (it votes across the warp); lanes past the end idle
         int t = base + threadIdx.x;
@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(BLOCK) k_build(RingArgs A)
         if (act) {
             if (A.worklist) {
                 pid = A.worklist[t];
+                if (pid < 0) pid = ~pid;   // too large a scan for the first stage
                 slot = A.slot_of[pid];
             } else {
                 slot = A.item_base + t;
@@ -429,10 +430,6 @@ __global__ void __launch_bounds__(WARP_KERNEL_WARPS * 32, 2) k_build_warp(RingAr
     const bool direct = A.worklist && item_count(A) <= A.warp_items;
     const int n = direct ? item_count(A) : min(*A.defer_count, A.npoints);
     const int *list = direct ? A.worklist : A.defer_list;
-    if (direct && A.repair && blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
-        atomicAdd(&A.st->repaired, (unsigned long long)n);
-        atomicMax(&A.st->rounds, A.round + 1);
-    }
     for (int item = blockIdx.x * WARP_KERNEL_WARPS + wib; item < n; item += gridDim.x * WARP_KERNEL_WARPS) {
         const int e = list[item];
         const int pid = e < 0 ? ~e : e;
@@ -674,6 +671,7 @@ static const int kShapeBlock[KERNEL_SHAPES] = { 64, 64, 64, 32, 32, 64, 64 };
 static const int kShapeLanes[KERNEL_SHAPES] = { 1, 1, 1, 1, 1, 4, 8 };
 
 int kernel_shape_cap(int shape) { return (shape >= 0 && shape < KERNEL_SHAPES) ? kShapeCap[shape] : -1; }
+int kernel_shape_lanes(int shape) { return (shape >= 0 && shape < KERNEL_SHAPES) ? kShapeLanes[shape] : -1; }
 int kernel_shape_block(int shape) { return (shape >= 0 && shape < KERNEL_SHAPES) ? kShapeBlock[shape] : -1; }
 
 cudaError_t launch_build(const RingArgs &a, int mode, int sms, int shape, cudaStream_t s)
@@ -753,7 +751,7 @@ __global__ void k_call_end(DevCtl *ctl, DevStatus *st, int rounds, int advance_s
     if (advance_step) ctl->step += 1;
     int f = st->err_flags;
     if (rounds > 0) {
-        if (st->list_count[rounds & 1] > 0) {
+        if ((rounds & 1 ? st->list_count1 : st->list_count0) > 0) {
             f |= EF_NOT_CONVERGED;
             st->err_flags |= EF_NOT_CONVERGED;
         }

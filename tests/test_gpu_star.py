@@ -1,0 +1,107 @@
+"""The first stage of builds and rebuilds (k_star) against the incremental kernels: a work
+budget below its scans leaves every point to them, and both must give the same arrays, for
+every form of input the first stage accepts (windows of every size, box edges, ragged and tiny
+sets, dense and sparse cells, both precisions, general boxes, batches, kept cell lists)."""
+import numpy as np
+import pytest
+
+from gpudelaunaytriangulation_b200 import workloads as W
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+HEX = (1.0, 0.5, 0.0, np.sqrt(3.0) / 2.0)
+
+
+def _rings(pts, box, cell, incremental, fp64=False, sizes=None, moved=None, stride=24):
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayBatch, DelaunayGPU
+
+    d = DelaunayBatch(sizes, box, stride, cell) if sizes is not None else DelaunayGPU(len(pts), stride, cell, box)
+    d.setPrecision(not fp64)
+    d.setCheckMode(True)
+    if incremental:
+        d.setWorkBudget(255)
+    P = torch.from_numpy(pts).cuda()
+    tri, nn = d.globalDelaunayTriangulation(P)
+    st = d.stats()
+    assert st["mismatches"] == 0 and st["error_flags"] & ~32 == 0, st
+    if moved is not None:
+        d.setFlipRepair(False)   # every flagged point through the rebuild rounds
+        P.copy_(torch.from_numpy(moved))
+        tri.view(len(pts), -1).masked_fill_(torch.arange(stride, device="cuda") >= nn[:, None], 0)
+        d.testAndRepairDelaunayTriangulation(P, tri, nn)
+        assert d.stats()["error_flags"] & ~32 == 0
+        tri.view(len(pts), -1).masked_fill_(torch.arange(stride, device="cuda") >= nn[:, None], 0)
+    return tri, nn
+
+
+def _same(*args, **kw):
+    a, b = _rings(*args, False, **kw), _rings(*args, True, **kw)
+    assert torch.equal(a[1], b[1])
+    assert torch.equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("n", [24, 63, 64, 65, 700, 19_999, 20_001, 150_000])
+@pytest.mark.parametrize("cell", [0.45, 0.8, 1.0, 1.3, 1.7, 2.6])
+def test_uniform_sets(n, cell):
+    L = float(np.sqrt(n))
+    _same(W.uniform_points(n, L, 500 + n), (L, L), cell)
+
+
+@pytest.mark.parametrize("aspect", [0.04, 0.3, 5.0])
+def test_rectangles(aspect):
+    n = 30_000
+    Lx, Ly = float(np.sqrt(n * aspect)), float(np.sqrt(n / aspect))
+    _same(W.uniform_points(n, Lx, 77, Ly), (Lx, Ly), 1.0)
+
+
+@pytest.mark.parametrize("jitter", [1e-7, 1e-4, 0.05])
+def test_lattices(jitter):
+    # collinear candidates at every angle, near-cocircular ones on every circle
+    pts, Lx, Ly = W.triangular_lattice(150, 150, jitter=jitter, seed=8)
+    _same(pts, (Lx, Ly), 1.0)
+
+
+@pytest.mark.parametrize("cell", [0.2, 0.5, 1.0])
+def test_clusters(cell):
+    pts, L = W.gaussian_mixture(60_000, components=12, sigma=3.0, L=260.0, seed=6)
+    _same(pts, (L, L), cell)
+
+
+@pytest.mark.parametrize("scale", [1e-9, 1e9])
+def test_float64_and_units(scale):
+    # the same set in other units: far from one, squares leave the filter's range
+    n = 25_000
+    L = float(np.sqrt(n))
+    pts = W.uniform_points(n, L, 91)
+    for fp64 in (False, True):
+        _same(pts, (L, L), 1.0, fp64=fp64)
+        _same(pts * scale, (L * scale, L * scale), scale, fp64=fp64)
+
+
+def test_general_box():
+    n = 25_000
+    s = float(np.sqrt(n / (np.sqrt(3.0) / 2.0)))
+    u = W.uniform_points(n, 1.0, 92)
+    m = np.array(HEX).reshape(2, 2) * s
+    for shift in (0.0, 3.0):   # outside the primary cell too
+        pts = np.ascontiguousarray((u + np.floor(shift * W.uniform_points(n, 1.0, 93))) @ m.T)
+        for fp64 in (False, True):
+            _same(pts, tuple(m.reshape(-1)), 1.0, fp64=fp64)
+
+
+def test_batch():
+    sizes = np.array([30, 5000, 0, 64, 40_000, 1000], dtype=np.int64)
+    boxes = np.stack([np.sqrt(np.maximum(sizes, 1).astype(np.float64))] * 2, axis=1)
+    pts = np.concatenate([W.uniform_points(int(k), float(L), 600 + i)
+                          for i, (k, L) in enumerate(zip(sizes, boxes[:, 0])) if k > 0])
+    _same(pts, boxes, 1.0, sizes=sizes)
+
+
+@pytest.mark.parametrize("sigma", [0.05, 0.3])
+@pytest.mark.parametrize("n", [900, 60_000])
+def test_rebuild_rounds(n, sigma):
+    # cell lists older than the positions, points across the box's edge among them
+    L = float(np.sqrt(n))
+    pts = W.uniform_points(n, L, 95)
+    _same(pts, (L, L), 1.0, moved=W.displace(pts, sigma, L, L, 96))
