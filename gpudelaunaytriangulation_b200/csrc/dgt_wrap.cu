@@ -384,10 +384,20 @@ struct Wrap {
             // (conditions and margins as in dgt_star.cu)
             bool good = g > ((T)0.001953125 / ((T)256 * PR::u() * PR::u())) * err1<T>(a) * err1<T>(b);
             const T ig = rcp_fast(g);
-            const float wx = (float)((b.y - a.y) * ig), wy = (float)((a.x - b.x) * ig);
-            const float hw = sqrt_over(wx * wx + wy * wy) * 1.00390625f;
+            float wx = (float)((b.y - a.y) * ig), wy = (float)((a.x - b.x) * ig);
+            float hw = sqrt_over(wx * wx + wy * wy) * 1.00390625f;
             good = good && hw < 1e15f;
             const bool in = lane < m;
+            if (in && !good) {
+                // a sliver: its circle in double
+                const double2 *P = IDX ? A.pos : A.spos;
+                const double2 oa = star_off<GEN>(P, &S, p, id), ob = star_off<GEN>(P, &S, p, M.id[kb]);
+                const double4 c = make_circ<double>(oa.x, oa.y, ob.x, ob.y);
+                wx = (float)c.x;
+                wy = (float)c.y;
+                hw = (float)(2.0 * c.w) * 1.00390625f;
+                good = c.w < 5e14;
+            }
             const bool all_good = __all_sync(FULL, !in || good);
             const bool real = __all_sync(FULL, !in || id >= 0);
             float u0 = 3e38f, u1 = -3e38f, v0 = 3e38f, v1 = -3e38f;
