@@ -110,6 +110,7 @@ struct dgt_context {
     int flip = 1;    // test-and-repair starts with edge flips (0: rebuild every flagged point)
     int graph_flip_rounds = ASYNC_FLIP_ROUNDS;   // flip rounds of unsynchronised calls
     bool binned = false;   // the cell lists hold a binning of the current grid
+    int star_small = 0;    // see RingArgs
     int flip_cap = 0;
     // global builds in this many pieces of the cell order, each on a stream of its own with
     // the points it defers (1: the whole build, then the deferred points)
@@ -316,6 +317,10 @@ int plan_grid(dgt_context *c)
         pbase += ns;
         if (cells > (1LL << 30)) return DGT_ERR_INVALID_ARGUMENT;
     }
+    // rows of a window in slots, half of the 16-bit range left for uneven densities
+    c->star_small = 1;
+    for (const SetDesc &S : c->sets)
+        if ((double)S.per_cell * S.xsize * (S.star_win / 2 + 1) > 16000.0) c->star_small = 0;
     c->total_cells = (int)cells;
     c->total_blocks = (int)blocks;
     return DGT_OK;
@@ -465,6 +470,7 @@ RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int str
     a.second_split = c->n / 4;   // 64-byte rings in 16 bytes a point
     a.second_cap = 2 * a.second_split;
     a.second_base = 0;
+    a.star_small = c->star_small;
     a.skin = &c->st.as<DevStatus>()->skin;
     a.work_budget = c->work_budget;
     a.check = c->check;

@@ -96,18 +96,27 @@ __device__ __forceinline__ int *second_ring(const RingArgs &A, int k)
                               : A.second_rings[1] + (size_t)(e - A.second_split) * STAR_RING;
 }
 
-template <typename T> struct StarMem {
+// Shared memory of a block, a column per thread.  SMALL (first pass with the float32 filter):
+// slots as 16-bit offsets from the point's own slot, so that 20 warps fit an SM instead of 16 (4M
+// uniform points: 1.49 -> 1.33 ms); for sets whose windows span fewer than 32,768 slots.
+template <typename T, bool SMALL> struct StarMem {
     typedef typename Prec<T>::T2 V2;
-    V2 q[STAR_CAP + 1][STAR_BLOCK];    // inverted offsets (the last: the stack's sentinel); the finished ring's indices
-    int s[STAR_CAP][STAR_BLOCK];       // slot (build) or index (repair) of a candidate; row starts from the end
+    static constexpr int B = SMALL ? 128 : STAR_BLOCK;
+    V2 q[SMALL ? STAR_CAP : STAR_CAP + 1][B];   // inverted offsets, behind them the stack's sentinel; the finished ring's indices
+    int s[SMALL ? STAR_CAP / 2 : STAR_CAP][B];  // slot (build) or index (repair) of a candidate
     // the sorted order, and the hull stack in its place: candidate numbers, the sentinel's first
     // and the first candidate's again at the end
-    unsigned char o[STAR_CAP + 4][STAR_BLOCK];
+    unsigned char o[STAR_CAP + 2][B];
+    // row ranges until they are taken: their starts, from the end of an array that fills from the front
+    __device__ __forceinline__ int &start(int k, int t)
+    {
+        return SMALL ? *reinterpret_cast<int *>(&q[STAR_CAP - k][t]) : s[SMALL ? 0 : STAR_CAP - k][t];
+    }
 };
 
-template <typename T>
+template <typename T, bool SMALL>
 struct StarRing {
-    StarMem<T> &M;
+    StarMem<T, SMALL> &M;
     int t;
     __device__ __forceinline__ int idx(int k) const { return *reinterpret_cast<const int *>(&M.q[k][t]); }
     __device__ __forceinline__ void set(int k, int v) { *reinterpret_cast<int *>(&M.q[k][t]) = v; }
@@ -121,8 +130,8 @@ struct StarRing {
 // segment to a'; d' lies within 2.7e-4 |d'| of that segment.  So d' is interior, and d is
 // dropped, if wmax |d'| < 3.6, which certify() checks.  Other pairs hand the point on.
 // Returns the candidates left (-1: hand on); drop: the largest |d'|^2 of those dropped.
-template <typename T>
-__device__ __noinline__ int settle_angles(StarMem<T> *M, int t, int n, unsigned close, bool wrap, T *drop)
+template <typename T, bool SMALL>
+__device__ __noinline__ int settle_angles(StarMem<T, SMALL> *M, int t, int n, unsigned close, bool wrap, T *drop)
 {
     auto at = [&](int k) { return &M->o[k + 1][t]; };
     auto len2 = [&](int k) { return M->q[k][t].x * M->q[k][t].x + M->q[k][t].y * M->q[k][t].y; };
@@ -154,13 +163,13 @@ __device__ __noinline__ int settle_angles(StarMem<T> *M, int t, int n, unsigned 
     return out;
 }
 
-template <typename T, bool IDX, bool GEN>
+template <typename T, bool IDX, bool GEN, bool SMALL, bool CHECK>
 struct Star {
     typedef Prec<T> PR;
     typedef typename PR::T2 V2;
     const RingArgs &A;
     const SetDesc &S;
-    StarMem<T> &M;
+    StarMem<T, SMALL> &M;
     const int t;
     double2 p;
     int self;        // own slot (build) or index (repair)
@@ -171,9 +180,10 @@ struct Star {
     int x0 = 0, x1 = 0, y0 = 0, y1 = 0, nseg = 0, total = 0;
     unsigned long long c0 = 0, c1 = 0;
     int n = 0, m = 0;
+    int spare = 0;   // SMALL: the place behind the candidates gathered
     unsigned cand = 0, tests = 0, u32 = 0, u64 = 0, ins = 0, mism = 0, cells = 0;
 
-    __device__ Star(const RingArgs &a, const SetDesc &s, StarMem<T> &mm, double2 pp, int self_)
+    __device__ Star(const RingArgs &a, const SetDesc &s, StarMem<T, SMALL> &mm, double2 pp, int self_)
         : A(a), S(s), M(mm), t(threadIdx.x), p(pp), self(self_)
     {
         const double2 f = cell_pos<GEN>(S, p);
@@ -183,6 +193,15 @@ struct Star {
         fy = f.y - (double)ocy;
     }
 
+    // the candidate at place k
+    __device__ __forceinline__ int slot(int k) const
+    {
+        if (!SMALL) return M.s[SMALL ? 0 : k][t];
+        int v = self + reinterpret_cast<const short *>(&M.s[SMALL ? k >> 1 : 0][t])[k & 1];
+        if (v < S.point_base) v += S.n;
+        else if (v >= S.point_base + S.n) v -= S.n;
+        return v;
+    }
     // candidate number k of the order / of the ring (the sentinel is number -1)
     __device__ __forceinline__ int ord(int k) { return M.o[k + 1][t]; }
     // W cells per axis: centred on the own cell (odd W), or on its half that holds p (even W)
@@ -207,9 +226,17 @@ struct Star {
             nseg = STAR_SEGS + 1;
             return;
         }
+        if (SMALL) {
+            // the offsets from the own slot must fit 16 bits (around the set: a window over its seam)
+            const int d = abs(s - self), e = min(d, S.n - d);
+            if (e + c > 32767) {
+                nseg = STAR_SEGS + 1;
+                return;
+            }
+        }
         // a stack: starts from the end of the candidate array down, counts in the 120-bit c1:c0
         ++nseg;
-        M.s[STAR_CAP - nseg][t] = s;
+        M.start(nseg, t) = s;
         c1 = (c1 << 10) | (c0 >> 50);
         c0 = ((c0 << 10) & ((1ull << 60) - 1ull)) | (unsigned)c;
     }
@@ -225,7 +252,7 @@ struct Star {
         if (xa < 0) xa += S.xsize;
         if (xb >= S.xsize) xb -= S.xsize;
         if (!seam) {
-#pragma unroll 4
+#pragma unroll 1
             for (int r = y0; r <= y1; ++r) {
                 const int cy = wrapi(ocy + r, S.ysize);
                 add_seg(cy, xa, cy, xb);
@@ -260,8 +287,9 @@ struct Star {
         // The ranges are taken from the last (lowest start word) on.  Without a cut the total fits
         // and every range left holds a candidate at least, so a candidate never reaches the words
         // of the ranges still to come; else the capacity leaves them alone.
-        const int cap = total <= STAR_CAP ? STAR_CAP - nw : STAR_CAP - max(nw, nseg);
-        int seg = nseg, left = 0, sl = 0, id = -1;
+        // (SMALL leaves a place for the sentinel; the point itself is in the total)
+        const int cap = total <= STAR_CAP ? STAR_CAP - nw - (SMALL ? 1 : 0) : STAR_CAP - max(nw, nseg);
+        int seg = nseg, left = 0, sl = 0, id = -1, shift = self;
         double2 c = make_double2(0.0, 0.0);
         // the next candidate's position is loaded a step ahead of its use
         auto next = [&]() {
@@ -270,7 +298,13 @@ struct Star {
                     id = -1;
                     return;
                 }
-                sl = M.s[STAR_CAP - seg][t];
+                sl = M.start(seg, t);
+                if (SMALL && WRAP) {
+                    // the nearest way round the set's slots
+                    shift = self;
+                    if (2 * (sl - self) > S.n) shift += S.n;
+                    else if (2 * (sl - self) < -S.n) shift -= S.n;
+                }
                 --seg;
                 left = (int)(c0 & 1023u);
                 c0 = (c0 >> 10) | ((c1 & 1023u) << 50);
@@ -283,7 +317,7 @@ struct Star {
         };
         next();
         while (id >= 0) {
-            const int cur = id;
+            const int cur = id, off = id - shift;
             double2 d64;
             if (GEN) d64 = gen_off(c, p, S);
             else if (WRAP) d64 = make_double2(wrap_off(c.x, p.x, S.Lx, S.hLx), wrap_off(c.y, p.y, S.Ly, S.hLy));
@@ -308,7 +342,8 @@ struct Star {
             }
             const T iv = rcp_fast(nd);
             M.q[n][t] = PR::mk2(dx * iv, dy * iv);
-            M.s[n][t] = cur;
+            if (SMALL) reinterpret_cast<short *>(&M.s[SMALL ? n >> 1 : 0][t])[n & 1] = (short)off;
+            else M.s[SMALL ? 0 : n][t] = cur;
             if (nd < ndmin) {
                 ndmin = nd;
                 near = n;
@@ -350,7 +385,7 @@ struct Star {
             if (k > 0 && k < n && key[k] - key[k > 0 ? k - 1 : 0] - 1u < STAR_ANGLE_TOL) close |= 1u << k;
         }
         T drop = (T)0;
-        n = settle_angles<T>(&M, t, n, close, 0u - last - 1u <= STAR_ANGLE_TOL, &drop);
+        n = settle_angles<T, SMALL>(&M, t, n, close, 0u - last - 1u <= STAR_ANGLE_TOL, &drop);
         dropped = drop;
         if (n < 3) status = S_FAIL;
     }
@@ -358,7 +393,7 @@ struct Star {
     // the float64 answer (for candidates at these places): +1 left, -1 right, 0 undecided
     __device__ __forceinline__ int recheck(int ka, int kb, int kc)
     {
-        return star_recheck<GEN, false>(IDX ? A.pos : A.spos, &S, p, M.s[ka][t], M.s[kb][t], M.s[kc][t]);
+        return star_recheck<GEN, false>(IDX ? A.pos : A.spos, &S, p, slot(ka), slot(kb), slot(kc));
     }
 
     // Graham pass over the sorted candidates, the stack in place of the order: the ring is
@@ -371,8 +406,9 @@ struct Star {
         if (status != S_TODO) return;   // a finished lane keeps its ring
         const int first = ord(0);
         V2 b = M.q[first][t], a = PR::mk2(-b.x, -b.y);
-        M.q[STAR_CAP][t] = a;
-        M.o[0][t] = (unsigned char)STAR_CAP;
+        const int sentinel = SMALL ? spare : STAR_CAP;
+        M.q[sentinel][t] = a;
+        M.o[0][t] = (unsigned char)sentinel;
         M.o[n + 1][t] = (unsigned char)first;
         int top = 0, i = 1, ci = ord(1);
         V2 c = M.q[ci][t];
@@ -382,7 +418,7 @@ struct Star {
             T o, bnd;
             turn<T>(a, b, c, ea, eb, ec, o, bnd);
             pop = o < -bnd;
-            if (A.check && pop && top > 0) mism += recheck(ord(top - 1), ord(top), ci) > 0;
+            if (CHECK && pop && top > 0) mism += recheck(ord(top - 1), ord(top), ci) > 0;
             if (pop ? top == 0 : i >= n) break;
             // one load serves both: the candidate below the new top, or the next in the order
             const int e = ord(pop ? top - 2 : i + 1);
@@ -449,7 +485,7 @@ struct Star {
             eb = ec;
         }
         // turns of the ring the filter left open: in float64
-        if (A.check) unsure = m == 32 ? ~0u : (1u << m) - 1u;
+        if (CHECK) unsure = m == 32 ? ~0u : (1u << m) - 1u;
         if (good && unsure) good = settle_turns(unsure);
         if (!good || !(wmax < (T)1e15) || (dropped > (T)0 && !(wmax * wmax * dropped < (T)8))) {
             status = S_FAIL;
@@ -476,7 +512,7 @@ struct Star {
             status = S_HEAVY;
             return;
         }
-        if (leave) return;
+        if (SMALL || leave) return;
         x0 = (int)floor(a0);
         x1 = (int)floor(a1);
         y0 = (int)floor(b0);
@@ -490,12 +526,12 @@ struct Star {
         for (int k = 0; k < m; ++k) {
             const V2 c = M.q[ord(k + 1 < m ? k + 1 : 0)][t];
             const T ig = rcp_fast(a.x * c.y - a.y * c.x);
-            M.s[2 * k][t] = __float_as_int((float)((c.y - a.y) * ig));
-            M.s[2 * k + 1][t] = __float_as_int((float)((a.x - c.x) * ig));
+            M.s[SMALL ? 0 : 2 * k][t] = __float_as_int((float)((c.y - a.y) * ig));
+            M.s[SMALL ? 0 : 2 * k + 1][t] = __float_as_int((float)((a.x - c.x) * ig));
             a = c;
         }
         for (int k = 0; k < m; ++k)
-            M.q[STAR_CAP - 1 - k][t] = PR::mk2((T)__int_as_float(M.s[2 * k][t]), (T)__int_as_float(M.s[2 * k + 1][t]));
+            M.q[STAR_CAP - 1 - k][t] = PR::mk2((T)__int_as_float(M.s[SMALL ? 0 : 2 * k][t]), (T)__int_as_float(M.s[SMALL ? 0 : 2 * k + 1][t]));
     }
 
     // ring vertices whose turns are unsure: all left in float64?
@@ -579,6 +615,7 @@ struct Star {
             // a safe range for squares and reciprocals, and enough for a ring
             if (status == S_TODO && (n < 3 || !(ndmin > (T)1e-30) || !(ndmax < (T)1e30))) status = S_FAIL;
         }
+        if (SMALL) spare = min(n, STAR_CAP - 1);
         __syncwarp();
         sort(near, dropped);
         __syncwarp();
@@ -623,16 +660,17 @@ struct Star {
             M.q[k][t] = PR::mk2(dx * iv, dy * iv);
         }
         for (int k = 0; k < m; ++k) {
-            M.s[k][t] = row[k];
+            M.s[SMALL ? 0 : k][t] = row[k];
             M.o[k + 1][t] = (unsigned char)k;
         }
     }
 };
 
-template <typename T, int MODE, bool IDX, bool GEN>
-__global__ void __launch_bounds__(STAR_BLOCK) k_star(RingArgs A)
+template <typename T, int MODE, bool IDX, bool GEN, bool SMALL, bool CHECK>
+__global__ void __launch_bounds__(SMALL ? 128 : STAR_BLOCK) k_star(RingArgs A)
 {
-    __shared__ StarMem<T> M;
+    __shared__ StarMem<T, SMALL> M;
+    constexpr int B = StarMem<T, SMALL>::B;
     const int t = threadIdx.x;
     Ctr ctr = { 0, 0, 0, 0, 0, 0, 0 };
     unsigned pts = 0;
@@ -643,7 +681,7 @@ __global__ void __launch_bounds__(STAR_BLOCK) k_star(RingArgs A)
         atomicMax(&A.st->rounds, A.round + 1);
     }
     if (IDX && n <= A.wrap_items) return;   // a short list: k_wrap takes it
-    for (int base = blockIdx.x * STAR_BLOCK; base < n; base += gridDim.x * STAR_BLOCK) {
+    for (int base = blockIdx.x * B; base < n; base += gridDim.x * B) {
         const int it = base + t;
         const bool act = it < n;
         int pid = -1, slot = -1;
@@ -653,17 +691,25 @@ __global__ void __launch_bounds__(STAR_BLOCK) k_star(RingArgs A)
         }
         const SetDesc &S = A.sets[(act && A.set_of) ? __ldg(&A.set_of[IDX ? pid : slot]) : 0];
         const double2 p = !act ? make_double2(0.0, 0.0) : (IDX ? __ldg(&A.pos[pid]) : __ldg(&A.spos[slot]));
-        Star<T, IDX, GEN> b(A, S, M, p, IDX ? pid : slot);
+        Star<T, IDX, GEN, SMALL, CHECK> b(A, S, M, p, IDX ? pid : slot);
         if (act && !IDX) pid = __ldg(&A.sidx[slot]);
         if (MODE == STAR_SECOND && act) b.load_ring(second_ring(A, it));
         b.run(MODE, act);
         if (act) {
-            StarRing<T> ring{ M, t };
+            StarRing<T, SMALL> ring{ M, t };
             if (b.status == S_OK) {
                 pts++;
-                for (int k = 0; k < b.m; ++k) {
-                    const int e = M.s[b.ord(k)][t];
-                    ring.set(k, IDX ? e : __ldg(&A.sidx[e]));
+                // (four loads in flight: 4M uniform points 1.68 -> 1.61 ms)
+                for (int k = 0; k < b.m; k += 4) {
+                    int e[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) e[j] = b.slot(k + j < b.m ? b.ord(k + j) : b.ord(k));
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (!IDX) e[j] = __ldg(&A.sidx[e[j]]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (k + j < b.m) ring.set(k + j, e[j]);
                 }
                 if (IDX) finish_repair(A, pid, ring, b.m);
                 store_ring(A, pid, ring, b.m, maxr);
@@ -675,7 +721,7 @@ __global__ void __launch_bounds__(STAR_BLOCK) k_star(RingArgs A)
                     A.second_list[at] = slot;
                     int *row = second_ring(A, at);
                     row[0] = b.m;
-                    for (int k = 0; k < b.m; ++k) row[k + 1] = M.s[b.ord(k)][t];
+                    for (int k = 0; k < b.m; ++k) row[k + 1] = b.slot(b.ord(k));
                 } else {
                     A.star_list[atomicAdd(A.star_count, 1)] = b.status == S_FAIL ? pid : ~pid;
                 }
@@ -693,13 +739,15 @@ __global__ void __launch_bounds__(STAR_BLOCK) k_star(RingArgs A)
     flush_counters(A, ctr, pts, maxr);
 }
 
-template <typename T, int MODE, bool IDX, bool GEN>
+template <typename T, int MODE, bool IDX, bool GEN, bool SMALL>
 cudaError_t launch_star_t(const RingArgs &a, int sms, cudaStream_t s)
 {
-    int blocks = (a.n_items + STAR_BLOCK - 1) / STAR_BLOCK;
-    const int most = sms * 8;
+    constexpr int B = StarMem<T, SMALL>::B;
+    int blocks = (a.n_items + B - 1) / B;
+    const int most = sms * (SMALL ? 5 : 8);
     if (blocks > most) blocks = most;
-    k_star<T, MODE, IDX, GEN><<<blocks, STAR_BLOCK, 0, s>>>(a);
+    if (a.check) k_star<T, MODE, IDX, GEN, SMALL, true><<<blocks, B, 0, s>>>(a);
+    else k_star<T, MODE, IDX, GEN, SMALL, false><<<blocks, B, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -707,11 +755,13 @@ template <typename T, bool GEN>
 cudaError_t launch_star_g(const RingArgs &a, int sms, int *launches, cudaStream_t s)
 {
     *launches += 1;
-    if (a.cand_by_index) return launch_star_t<T, STAR_BOTH, true, GEN>(a, sms, s);
-    cudaError_t e = launch_star_t<T, STAR_FIRST, false, GEN>(a, sms, s);
+    if (a.cand_by_index) return launch_star_t<T, STAR_BOTH, true, GEN, false>(a, sms, s);
+    cudaError_t e;
+    if (sizeof(T) == 4 && a.star_small) e = launch_star_t<T, STAR_FIRST, false, GEN, sizeof(T) == 4>(a, sms, s);
+    else e = launch_star_t<T, STAR_FIRST, false, GEN, false>(a, sms, s);
     if (e != cudaSuccess) return e;
     *launches += 1;
-    return launch_star_t<T, STAR_SECOND, false, GEN>(a, sms, s);
+    return launch_star_t<T, STAR_SECOND, false, GEN, false>(a, sms, s);
 }
 
 }  // namespace

@@ -13,12 +13,12 @@ pytestmark = pytest.mark.gpu
 HEX = (1.0, 0.5, 0.0, np.sqrt(3.0) / 2.0)
 
 
-def _rings(pts, box, cell, incremental, fp64=False, sizes=None, moved=None, stride=24):
+def _rings(pts, box, cell, incremental, fp64=False, sizes=None, moved=None, stride=24, check=False):
     from gpudelaunaytriangulation_b200.delaunay import DelaunayBatch, DelaunayGPU
 
     d = DelaunayBatch(sizes, box, stride, cell) if sizes is not None else DelaunayGPU(len(pts), stride, cell, box)
     d.setPrecision(not fp64)
-    d.setCheckMode(True)
+    d.setCheckMode(check)
     if incremental:
         d.setWorkBudget(255)
     P = torch.from_numpy(pts).cuda()
@@ -36,9 +36,11 @@ def _rings(pts, box, cell, incremental, fp64=False, sizes=None, moved=None, stri
 
 
 def _same(*args, **kw):
-    a, b = _rings(*args, False, **kw), _rings(*args, True, **kw)
-    assert torch.equal(a[1], b[1])
-    assert torch.equal(a[0], b[0])
+    b = _rings(*args, True, **kw)
+    for check in (False, True):   # (check mode: every decision contradicted by float64 is counted)
+        a = _rings(*args, False, check=check, **kw)
+        assert torch.equal(a[1], b[1])
+        assert torch.equal(a[0], b[0])
 
 
 @pytest.mark.parametrize("n", [24, 63, 64, 65, 700, 19_999, 20_001, 150_000])
