@@ -26,6 +26,7 @@
 //
 // Angles.  r = y / (|x| + |y|) continued over the four quadrants has an error of at most 16u =
 // two units of 2^-21; keys whose difference exceeds four units are in their true order.
+#include <type_traits>
 #include "dgt_star.cuh"
 
 namespace dgt {
@@ -103,14 +104,15 @@ template <typename T, bool SMALL> struct StarMem {
     typedef typename Prec<T>::T2 V2;
     static constexpr int B = SMALL ? 128 : STAR_BLOCK;
     V2 q[SMALL ? STAR_CAP : STAR_CAP + 1][B];   // inverted offsets, behind them the stack's sentinel; the finished ring's indices
-    int s[SMALL ? STAR_CAP / 2 : STAR_CAP][B];  // slot (build) or index (repair) of a candidate
+    typedef typename std::conditional<SMALL, short, int>::type Slot;
+    Slot s[STAR_CAP][B];  // slot (build) or index (repair) of a candidate
     // the sorted order, and the hull stack in its place: candidate numbers, the sentinel's first
     // and the first candidate's again at the end
     unsigned char o[STAR_CAP + 2][B];
     // row ranges until they are taken: their starts, from the end of an array that fills from the front
     __device__ __forceinline__ int &start(int k, int t)
     {
-        return SMALL ? *reinterpret_cast<int *>(&q[STAR_CAP - k][t]) : s[SMALL ? 0 : STAR_CAP - k][t];
+        return SMALL ? *reinterpret_cast<int *>(&q[STAR_CAP - k][t]) : *reinterpret_cast<int *>(&s[STAR_CAP - k][t]);
     }
 };
 
@@ -196,8 +198,8 @@ struct Star {
     // the candidate at place k
     __device__ __forceinline__ int slot(int k) const
     {
-        if (!SMALL) return M.s[SMALL ? 0 : k][t];
-        int v = self + reinterpret_cast<const short *>(&M.s[SMALL ? k >> 1 : 0][t])[k & 1];
+        if (!SMALL) return M.s[k][t];
+        int v = self + M.s[k][t];
         if (v < S.point_base) v += S.n;
         else if (v >= S.point_base + S.n) v -= S.n;
         return v;
@@ -342,8 +344,7 @@ struct Star {
             }
             const T iv = rcp_fast(nd);
             M.q[n][t] = PR::mk2(dx * iv, dy * iv);
-            if (SMALL) reinterpret_cast<short *>(&M.s[SMALL ? n >> 1 : 0][t])[n & 1] = (short)off;
-            else M.s[SMALL ? 0 : n][t] = cur;
+            M.s[n][t] = SMALL ? off : cur;
             if (nd < ndmin) {
                 ndmin = nd;
                 near = n;
@@ -405,6 +406,36 @@ struct Star {
     {
         if (status != S_TODO) return;   // a finished lane keeps its ring
         const int first = ord(0);
+        if (!CHECK) {
+            // A pass without a stack first: a candidate at a certain right turn between the last one
+            // kept and the next one is interior.  It drops more than half of them at half the
+            // instructions that the pass with the stack spends on one (4M uniform points: 1.42 ->
+            // 1.28 ms; a second such pass gains nothing, and unrolled over the sorted keys it lost 6%
+            // to instruction fetch).  Check mode leaves every decision to the loop that counts them.
+            M.o[n + 1][t] = (unsigned char)first;
+            int kept = 0, cur = ord(1);
+            V2 a = M.q[first][t], b = M.q[cur][t];
+            T ea = err1<T>(a), eb = err1<T>(b);
+#pragma unroll 1
+            for (int k = 1; k < n; ++k) {
+                const int next = ord(k + 1);
+                const V2 c = M.q[next][t];
+                const T ec = err1<T>(c);
+                T o, bnd;
+                turn<T>(a, b, c, ea, eb, ec, o, bnd);
+                if (!(o < -bnd)) {
+                    ++kept;
+                    M.o[kept + 1][t] = (unsigned char)cur;
+                    a = b;
+                    ea = eb;
+                }
+                b = c;
+                eb = ec;
+                cur = next;
+            }
+            tests += (unsigned)(n - 1);
+            n = kept + 1;
+        }
         V2 b = M.q[first][t], a = PR::mk2(-b.x, -b.y);
         const int sentinel = SMALL ? spare : STAR_CAP;
         M.q[sentinel][t] = a;
