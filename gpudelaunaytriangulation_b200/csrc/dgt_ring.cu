@@ -485,31 +485,9 @@ __device__ __forceinline__ void warp_append(int *list, int *count, const int *it
 constexpr int TEST_MAX_QUEUE = 24;
 constexpr int TEST_MAX_EDGES = 6;
 
-__device__ __forceinline__ void warp_append_edges(int2 *list, int *count, int cap, const int2 *items, int k,
-                                                  int *overflow)
-{
-    const int lane = threadIdx.x & 31;
-    int incl = k;
-    for (int o = 1; o < 32; o <<= 1) {
-        int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    int total = __shfl_sync(0xffffffffu, incl, 31);
-    int base = 0;
-    if (lane == 31 && total > 0) base = atomicAdd(count, total);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    int off = base + incl - k;
-    *overflow = 0;
-    for (int i = 0; i < k; ++i) {
-        if (off + i < cap) list[off + i] = items[i];
-        else *overflow = 1;
-    }
-}
-
 // One spoke (p, P_k) of a fan: triangle (p, P_k, P_k+1) strictly CCW and P_k+1 outside the
 // circle through (p, P_k-1, P_k); counts the winding crossing and records failures
-__device__ __forceinline__ void test_spoke(double2 prev, double2 cur, double2 nxt, int k, int rk, int i, bool flip,
-                                           int &cross, int &nf, int *fail_k, bool &inverted, int2 *ev, int &ne)
+__device__ __forceinline__ void test_spoke(double2 prev, double2 cur, double2 nxt, int k, int &cross, int &nf, int *fail_k)
 {
     int o = orient32(__double2float_rn(cur.x), __double2float_rn(cur.y), __double2float_rn(nxt.x),
                      __double2float_rn(nxt.y));
@@ -522,16 +500,9 @@ __device__ __forceinline__ void test_spoke(double2 prev, double2 cur, double2 nx
         if (nf < 3) fail_k[nf] = k;
         nf++;
     }
-    inverted |= o <= 0;
-    if (flip && o > 0 && ic >= 0 && i < rk) {
-        if (ne < TEST_MAX_EDGES) ev[ne] = make_int2(i, rk);
-        ne++;
-    }
 }
 
-// Flip mode (A.flip_list set): a valid fan (every triangle strictly CCW, winding once) sends
-// its illegal or undecided spokes (i, P_k) with i < P_k to the flip list (the flip stage
-// decides them exactly); an invalid fan queues its point for rebuilding.
+// (rebuild-only mode; k_test_flip is the flip mode's)
 // four blocks per SM (64 registers): more warps in flight hide the neighbour gathers
 // (measured: -4% repair time against three blocks at 73 registers)
 template <bool GEN>
@@ -539,28 +510,13 @@ __global__ void __launch_bounds__(256, 4) k_test(TestArgs A)
 {
     unsigned long long flagged = 0;
     const int ebase = *A.epoch_ptr + 1;
-    const bool flip = A.flip_list != nullptr;
-    float moved = 0.0f;   // largest distance outside the listing cell (when A.rcell_of is set)
     for (int base = blockIdx.x * blockDim.x; base < A.n; base += gridDim.x * blockDim.x) {
         // points taken in cell order (slot t -> point sidx[t]): the queue a warp appends is a
         // compact patch of cells, which keeps the repair rounds spatially coherent
-        // flip mode: index order (rows, ring lengths and owner positions stream contiguously;
-        // only the neighbour gathers are random)
         const int t = base + threadIdx.x;
-        const int i = (t < A.n && A.sidx && !flip) ? A.sidx[t] : t;
+        const int i = t < A.n ? A.sidx[t] : t;
         int q[TEST_MAX_QUEUE];
         int nq = 0;
-        int2 ev[TEST_MAX_EDGES];
-        int ne = 0;
-        bool inverted = false;
-        if (t < A.n && A.rcell_of) {
-            const SetDesc S = A.sets[A.set_of ? A.set_of[i] : 0];
-            const double2 p = A.pos[i];
-            const bool bad_in = GEN ? !(isfinite(p.x) && isfinite(p.y))
-                                    : !(p.x >= 0.0 && p.x < S.Lx && p.y >= 0.0 && p.y < S.Ly);
-            if (bad_in) atomicOr(&A.st->err_flags, EF_BAD_INPUT);
-            moved = fmaxf(moved, outside_cell<GEN>(S, A.rcell_of[i], p));
-        }
         if (t < A.n) {
             int m = A.nn[i];
             bool bad = (m < 3 || m > A.stride);
@@ -574,7 +530,7 @@ __global__ void __launch_bounds__(256, 4) k_test(TestArgs A)
                 }
                 if (!bad) {
                 const SetDesc S = A.sets[A.set_of ? A.set_of[i] : 0];
-                double2 p = (A.sidx && !flip) ? A.spos[t] : A.pos[i];
+                double2 p = A.spos[t];
                 double2 q0 = __ldg(&A.pos[row[0]]), ql = __ldg(&A.pos[row[m - 1]]);
                 double2 o0 = GEN ? gen_off(q0, p, S)
                                  : make_double2(wrap_off(q0.x, p.x, S.Lx, S.hLx), wrap_off(q0.y, p.y, S.Ly, S.hLy));
@@ -595,20 +551,14 @@ __global__ void __launch_bounds__(256, 4) k_test(TestArgs A)
                     } else {
                         nxt = o0;
                     }
-                    test_spoke(prev, cur, nxt, k, row[k], i, flip, cross, nf, fail_k, inverted, ev, ne);
+                    test_spoke(prev, cur, nxt, k, cross, nf, fail_k);
                     prev = cur;
                     cur = nxt;
                 }
                 if (cross != 1) bad = true;
                 }
             }
-            if (flip) {
-                // invalid fan (or more illegal spokes than the edge buffer): rebuild the point
-                if (bad || inverted || ne > TEST_MAX_EDGES) {
-                    if (atomicMax(&A.mark[i], ebase) < ebase) q[nq++] = i;
-                    ne = 0;
-                }
-            } else if (bad || nf > 0) {
+            if (bad || nf > 0) {
                 if (atomicMax(&A.mark[i], ebase) < ebase) q[nq++] = i;
                 if (!bad) {
                     // a spoke failure: its quadrilateral; more than three failures: the whole fan
@@ -629,18 +579,193 @@ __global__ void __launch_bounds__(256, 4) k_test(TestArgs A)
             }
         }
         flagged += nq;
-        if (flip) {
-            int overflow = 0;
-            warp_append_edges(A.flip_list, A.flip_count, A.flip_cap, ev, ne, &overflow);
-            if (overflow && atomicMax(&A.mark[i], ebase) < ebase) {
-                q[nq++] = i;   // list full: the point's spokes are settled by rebuilding it
-                flagged++;
-            }
-        }
         warp_append(A.list, A.list_count, q, nq);
     }
     for (int o = 16; o > 0; o >>= 1) flagged += __shfl_down_sync(0xffffffffu, flagged, o);
     if ((threadIdx.x & 31) == 0 && flagged) atomicAdd(&A.st->flagged, flagged);
+}
+
+// Spokes of a fan the float32 filter leaves open, in float64: the orientation of the triangle
+// (i, P_k, P_k+1) and the in-circle of P_k+1 against (i, P_k-1, P_k)
+template <bool GEN>
+__device__ __noinline__ int2 test_spoke64(const double2 *pos, const SetDesc *S, double2 p, int ia, int ib, int ic)
+{
+    const double2 qa = pos[ia], qb = pos[ib], qc = pos[ic];
+    double2 a, b, c;
+    if (GEN) {
+        a = gen_off(qa, p, *S);
+        b = gen_off(qb, p, *S);
+        c = gen_off(qc, p, *S);
+    } else {
+        a = make_double2(wrap_off(qa.x, p.x, S->Lx, S->hLx), wrap_off(qa.y, p.y, S->Ly, S->hLy));
+        b = make_double2(wrap_off(qb.x, p.x, S->Lx, S->hLx), wrap_off(qb.y, p.y, S->Ly, S->hLy));
+        c = make_double2(wrap_off(qc.x, p.x, S->Lx, S->hLx), wrap_off(qc.y, p.y, S->Ly, S->hLy));
+    }
+    return make_int2(orient64(b.x, b.y, c.x, c.y), incircle64(a.x, a.y, b.x, b.y, c.x, c.y));
+}
+
+// float32 offset of q relative to p (the double offset, rounded)
+template <bool GEN>
+__device__ __forceinline__ float2 test_off(double2 q, double2 p, const SetDesc &S)
+{
+    double2 d;
+    if (GEN) {
+        d = gen_off(q, p, S);
+    } else {
+        // (one comparison per axis in the common case; the same value as wrap_off)
+        d = make_double2(__dsub_rn(q.x, p.x), __dsub_rn(q.y, p.y));
+        if (fabs(d.x) > S.hLx) d.x = wrap_off(q.x, p.x, S.Lx, S.hLx);
+        if (fabs(d.y) > S.hLy) d.y = wrap_off(q.y, p.y, S.Ly, S.hLy);
+    }
+    return make_float2(__double2float_rn(d.x), __double2float_rn(d.y));
+}
+
+// The test in flip mode, index order (rows, ring lengths and owner positions stream; only the
+// neighbour gathers are random): a valid fan (every triangle strictly CCW, winding once) sends
+// its illegal or undecided spokes (i, P_k) with i < P_k to the flip list (the flip stage decides
+// them exactly); an invalid fan, or one with more than TEST_MAX_EDGES such spokes, queues its
+// point for rebuilding.  Also measures how far the points left the cells that list them
+// (A.rcell_of).  What bounds it: instruction issue; the spokes share their products (the cross
+// product of P_k and P_k+1 serves the orientation and two in-circles), the row is read once and
+// the cell distance only computed for points that changed cell.
+// VEC: rows are 16-byte aligned and hold TEST_ROW entries at least
+constexpr int TEST_ROW = 8;
+template <bool GEN, bool VEC>
+__global__ void __launch_bounds__(256, 3) k_test_flip(TestArgs A)
+{
+    unsigned flagged = 0;
+    const int ebase = *A.epoch_ptr + 1;
+    float moved = 0.0f;
+    for (int base = blockIdx.x * blockDim.x; base < A.n; base += gridDim.x * blockDim.x) {
+        const int i = base + threadIdx.x;
+        unsigned fail = 0;   // bit k: spoke k goes to the flip list
+        bool rebuild = false;
+        const int *row = A.tri + (size_t)(i < A.n ? i : 0) * A.stride;
+        if (i < A.n) {
+            const SetDesc &S = A.sets[A.set_of ? __ldg(&A.set_of[i]) : 0];
+            const double2 p = __ldg(&A.pos[i]);
+            const int m = A.nn[i];
+            if (A.rcell_of) {
+                const bool bad_in = GEN ? !(isfinite(p.x) && isfinite(p.y))
+                                        : !(p.x >= 0.0 && p.x < S.Lx && p.y >= 0.0 && p.y < S.Ly);
+                if (bad_in) atomicOr(&A.st->err_flags, EF_BAD_INPUT);
+                const double2 f = cell_pos<GEN>(S, p);
+                const int cx = min(max((int)floor(f.x), 0), S.xsize - 1), cy = min(max((int)floor(f.y), 0), S.ysize - 1);
+                const int c = __ldg(&A.rcell_of[i]);
+                if (S.cell_base + cy * S.xsize + cx != c) moved = fmaxf(moved, outside_cell<GEN>(S, c, p));
+            }
+            bool bad = m < 3 || m > A.stride || m > 32;
+            if (!bad) {
+                // The first TEST_ROW entries with vector loads (a row is a cache line of its own for
+                // every lane, so each load of it costs as much as a neighbour's position), then
+                // their positions, all in flight together
+                auto valid = [&](int r) {
+                    const bool ok = (unsigned)r < (unsigned)A.n && r != i;
+                    bad |= !ok;
+                    return ok ? r : i;
+                };
+                int e[TEST_ROW];
+                if (VEC) {
+                    const int4 u = __ldg(reinterpret_cast<const int4 *>(row)), w = __ldg(reinterpret_cast<const int4 *>(row) + 1);
+                    e[0] = u.x, e[1] = u.y, e[2] = u.z, e[3] = u.w, e[4] = w.x, e[5] = w.y, e[6] = w.z, e[7] = w.w;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < TEST_ROW; ++k) e[k] = k < m ? row[k] : i;
+                }
+                double2 q[TEST_ROW];
+#pragma unroll
+                for (int k = 0; k < TEST_ROW; ++k) {
+                    e[k] = k < m ? valid(e[k]) : i;
+                    q[k] = k < m ? __ldg(&A.pos[e[k]]) : p;
+                }
+                float2 d[TEST_ROW];
+#pragma unroll
+                for (int k = 0; k < TEST_ROW; ++k) d[k] = test_off<GEN>(q[k], p, S);
+                float2 prev = d[0];
+                int rprev = e[0];
+                if (m > TEST_ROW) {
+                    rprev = valid(row[m - 1]);
+                    prev = test_off<GEN>(__ldg(&A.pos[rprev]), p, S);
+                } else {
+#pragma unroll
+                    for (int k = 1; k < TEST_ROW; ++k)
+                        if (k == m - 1) {
+                            prev = d[k];
+                            rprev = e[k];
+                        }
+                }
+                float2 cur = d[0];
+                int rcur = e[0];
+                float na = prev.x * prev.x + prev.y * prev.y, nb = cur.x * cur.x + cur.y * cur.y;
+                float g1 = prev.x * cur.y, g2 = prev.y * cur.x;
+                float gp = g1 - g2, gph = fabsf(g1) + fabsf(g2);   // prev x cur
+                int cross = 0;
+                bool inverted = false;
+                auto spoke = [&](int k, float2 nxt, int rnxt) {
+                    const float nd = nxt.x * nxt.x + nxt.y * nxt.y;
+                    g1 = cur.x * nxt.y;
+                    g2 = cur.y * nxt.x;
+                    const float gn = g1 - g2, gnh = fabsf(g1) + fabsf(g2);   // cur x next
+                    g1 = prev.x * nxt.y;
+                    g2 = prev.y * nxt.x;
+                    const float h = g1 - g2, hh = fabsf(g1) + fabsf(g2);     // prev x next
+                    // orient32 of (cur, next) and incircle32 of (prev, cur, next), with their bounds
+                    const float ob = 3.5762786865234375e-07f * gnh + 1e-30f;
+                    const float v = nb * h - na * gn - nd * gp;
+                    const float vb = 9.5367431640625e-07f * (na * gnh + nb * hh + nd * gph) + 1e-30f;
+                    bool ccw = gn > ob, outside = v < -vb;
+                    if ((!ccw && !(gn < -ob)) || (!outside && !(v > vb))) {
+                        const int2 t = test_spoke64<GEN>(A.pos, &S, p, rprev, rcur, rnxt);
+                        if (!ccw && !(gn < -ob)) ccw = t.x > 0;
+                        if (!outside && !(v > vb)) outside = t.y < 0;
+                    }
+                    cross += cur.y < 0.0f && nxt.y >= 0.0f;
+                    inverted |= !ccw;
+                    fail |= (unsigned)(!outside && i < rcur) << k;
+                    prev = cur;
+                    cur = nxt;
+                    na = nb;
+                    nb = nd;
+                    gp = gn;
+                    gph = gnh;
+                    rprev = rcur;
+                    rcur = rnxt;
+                };
+#pragma unroll
+                for (int k = 0; k + 1 < TEST_ROW; ++k)
+                    if (k < m) spoke(k, k + 1 == m ? d[0] : d[k + 1], k + 1 == m ? e[0] : e[k + 1]);
+                for (int k = TEST_ROW - 1; k < m; ++k) {
+                    const int r = k + 1 == m ? e[0] : valid(row[k + 1]);
+                    spoke(k, k + 1 == m ? d[0] : test_off<GEN>(__ldg(&A.pos[r]), p, S), r);
+                }
+                bad |= cross != 1 || inverted;
+            }
+            rebuild = bad || __popc(fail) > TEST_MAX_EDGES;
+            if (rebuild) fail = 0;
+        }
+        // the warp's failing spokes behind one another
+        const int lane = threadIdx.x & 31;
+        int k = __popc(fail), incl = k;
+        if (__any_sync(0xffffffffu, k > 0)) {
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            int at = 0;
+            if (lane == 31) at = atomicAdd(A.flip_count, incl);
+            at = __shfl_sync(0xffffffffu, at, 31) + incl - k;
+            for (; fail; fail &= fail - 1, ++at) {
+                if (at < A.flip_cap) A.flip_list[at] = make_int2(i, row[__ffs(fail) - 1]);
+                else rebuild = true;   // list full: the point's spokes are settled by rebuilding it
+            }
+        }
+        if (rebuild && atomicMax(&A.mark[i], ebase) < ebase) {
+            A.list[atomicAdd(A.list_count, 1)] = i;
+            ++flagged;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) flagged += __shfl_down_sync(0xffffffffu, flagged, o);
+    if ((threadIdx.x & 31) == 0 && flagged) atomicAdd(&A.st->flagged, (unsigned long long)flagged);
     for (int o = 16; o > 0; o >>= 1) moved = fmaxf(moved, __shfl_down_sync(0xffffffffu, moved, o));
     if ((threadIdx.x & 31) == 0 && moved > 0.0f)
         atomicMax(reinterpret_cast<int *>(&A.st->skin_measured), __float_as_int(moved));
@@ -705,8 +830,19 @@ cudaError_t launch_test(const TestArgs &a, cudaStream_t s)
 {
     if (a.n <= 0) return cudaSuccess;
     int blocks = (a.n + 255) / 256;
-    if (a.general) k_test<true><<<blocks, 256, 0, s>>>(a);
-    else k_test<false><<<blocks, 256, 0, s>>>(a);
+    if (a.flip_list) {
+        const bool vec = (a.stride & 3) == 0 && a.stride >= TEST_ROW && (reinterpret_cast<uintptr_t>(a.tri) & 15) == 0;
+        if (a.general) {
+            if (vec) k_test_flip<true, true><<<blocks, 256, 0, s>>>(a);
+            else k_test_flip<true, false><<<blocks, 256, 0, s>>>(a);
+        } else {
+            if (vec) k_test_flip<false, true><<<blocks, 256, 0, s>>>(a);
+            else k_test_flip<false, false><<<blocks, 256, 0, s>>>(a);
+        }
+    } else {
+        if (a.general) k_test<true><<<blocks, 256, 0, s>>>(a);
+        else k_test<false><<<blocks, 256, 0, s>>>(a);
+    }
     return cudaGetLastError();
 }
 
