@@ -407,16 +407,11 @@ BinArgs bin_args(dgt_context *c, const double *pts)
     return a;
 }
 
+// (clears the status first)
 cudaError_t run_bin(dgt_context *c, const double *pts, cudaStream_t s)
 {
     PhaseTimer t(c, DGT_PHASE_BIN, s);
-    cudaError_t e = cudaMemsetAsync(c->ccount.p, 0, sizeof(int) * ((size_t)c->total_cells + 1), s);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(c->bcount.p, 0, sizeof(int) * ((size_t)c->total_blocks + 1), s);
-    if (e != cudaSuccess) return e;
-    // count, super-block occupancy and scatter; three scan kernels; the in-cell order
-    c->launches += (c->n > 0 ? 3 : 0) + 3 + (c->deterministic && c->total_cells > 0 ? 1 : 0);
-    e = launch_bin_st(bin_args(c, pts), c->st.as<DevStatus>(), s);
+    cudaError_t e = launch_bin_all(bin_args(c, pts), c->st.as<DevStatus>(), true, &c->launches, s);
     if (e == cudaSuccess) c->binned = true;
     return e;
 }
@@ -432,11 +427,8 @@ cudaError_t run_bin_refresh(dgt_context *c, const double *pts, cudaStream_t s)
     cudaError_t e = launch_refresh(a, st, MAX_SKIN_CELLS, s);
     if (e != cudaSuccess) return e;
     a.cond = &st->rebin;
-    e = launch_clear_counts(c->ccount.as<int>(), c->total_cells + 1, c->bcount.as<int>(), c->total_blocks + 1,
-                            a.cond, s);
-    if (e != cudaSuccess) return e;
-    c->launches += (c->n > 0 ? 6 : 3) + 3 + (c->deterministic && c->total_cells > 0 ? 1 : 0);
-    return launch_bin_st(a, st, s);
+    c->launches += c->n > 0 ? 2 : 1;
+    return launch_bin_all(a, st, false, &c->launches, s);
 }
 
 RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int stride)
@@ -497,7 +489,11 @@ cudaError_t run_rings(dgt_context *c, const RingArgs &a, cudaStream_t s, PhaseTi
     if (c->work_budget >= STAR_MIN_BUDGET && kernel_shape_lanes(shape) == 1) {
         b.wrap_items = WRAP_REPAIR_MAX;
         b.wrap_mode = a.repair ? WRAP_REPAIR : (a.n_items <= WRAP_BUILD_MAX ? WRAP_OWN : WRAP_HANDED);
-        if (b.wrap_mode != WRAP_OWN && (e = launch_star(b, mode, c->sms, &c->launches, s)) != cudaSuccess) return e;
+        const bool short_lists = a.repair && a.n_items <= WRAP_REPAIR_MAX;   // (k_wrap takes them whole)
+        if (b.wrap_mode != WRAP_OWN && !short_lists) {
+            if ((e = launch_star(b, mode, c->sms, &c->launches, s)) != cudaSuccess) return e;
+            b.count_round = 0;
+        }
         if ((e = launch_wrap(b, mode, c->sms, s)) != cudaSuccess) return e;
         b.worklist = nullptr;
     } else {
@@ -578,10 +574,9 @@ void to_stats(const DevStatus &d, dgt_stats *o)
     o->error_flags = d.err_flags;
 }
 
-// read the device status (synchronising) and turn it into a status code
+// wait for the status that the call's end kernel left in host memory and turn it into a code
 int conclude(dgt_context *c, cudaStream_t s, bool repair_pending)
 {
-    DGT_TRY(cudaMemcpyAsync(c->h_st, c->st.p, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
     DGT_TRY(cudaStreamSynchronize(s));
     c->stats_valid = true;
     const DevStatus &d = *c->h_st;
@@ -742,7 +737,6 @@ int dgt_update_list(dgt_context *c, const double *d_points, void *stream)
 {
     if (!c || (c->n > 0 && !d_points)) return DGT_ERR_INVALID_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
-    DGT_TRY(cudaMemsetAsync(c->st.p, 0, sizeof(DevStatus), s));
     DGT_TRY(run_bin(c, d_points, s));
     c->last_stream = s;
     return DGT_OK;
@@ -756,7 +750,6 @@ int dgt_global_triangulation(dgt_context *c, const double *d_points, int *d_tri,
     if (!d_points || !d_tri || !d_nn || !valid_stride(stride)) return DGT_ERR_INVALID_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
     begin_call(c, s);
-    DGT_TRY(cudaMemsetAsync(c->st.p, 0, sizeof(DevStatus), s));
     DGT_TRY(run_bin(c, d_points, s));
     RingArgs a = ring_args(c, d_points, d_tri, d_nn, stride);
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -770,7 +763,7 @@ int dgt_global_triangulation(dgt_context *c, const double *d_points, int *d_tri,
         DGT_TRY(run_rings(c, a, s, &t));
     }
     c->launches += 1;
-    DGT_TRY(launch_call_end(c->ctl.as<DevCtl>(), c->st.as<DevStatus>(), 0, s));
+    DGT_TRY(launch_call_end(c->ctl.as<DevCtl>(), c->st.as<DevStatus>(), 0, s, false, false, c->safety ? c->h_st : nullptr));
     if (!c->safety) return DGT_OK;
     return conclude(c, s, false);
 }
@@ -840,6 +833,7 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
         DGT_TRY(launch_test(t, s));
     }
     phase_begin(c, DGT_PHASE_REPAIR, s);
+    bool skin_known = false;
     if (c->flip) {
         // Lawson flips first; what they cannot settle joins the rebuild list (list 0)
         FlipArgs f;
@@ -861,38 +855,44 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
         f.quad = c->quad.as<int2>();
         f.cap = c->flip_cap;
         f.st = dst;
-        int fr = 0;
-        for (;;) {
-            const int batch = fixed_rounds > 0 ? c->graph_flip_rounds : FLIP_BATCH;
-            for (int b = 0; b < batch; ++b, ++fr) {
-                f.cur = flips[fr & 1];
-                f.cur_count = &dst->flip_count[fr & 1];
-                f.next = flips[(fr + 1) & 1];
-                f.next_count = &dst->flip_count[(fr + 1) & 1];
-                c->launches += 2;
-                DGT_TRY(launch_flip_round(f, fr, c->sms, s));
+        const float max_skin = fold ? MAX_SKIN_CELLS : -1.0f;
+        int *counts[2] = { &dst->flip_count[0], &dst->flip_count[1] };
+        if (c->n <= FLIP_SMALL_MAX) {
+            c->launches += 1;
+            DGT_TRY(launch_flip_small(f, fixed_rounds > 0 ? c->graph_flip_rounds : MAX_FLIP_ROUNDS, ctl, flips, counts,
+                                      max_skin, s));
+        } else {
+            int fr = 0;
+            for (;;) {
+                const int batch = fixed_rounds > 0 ? c->graph_flip_rounds : FLIP_BATCH;
+                for (int b = 0; b < batch; ++b, ++fr) {
+                    f.cur = flips[fr & 1];
+                    f.cur_count = counts[fr & 1];
+                    f.next = flips[(fr + 1) & 1];
+                    f.next_count = counts[(fr + 1) & 1];
+                    c->launches += 2;
+                    DGT_TRY(launch_flip_round(f, fr, c->sms, s));
+                }
+                if (fixed_rounds > 0 || fr >= MAX_FLIP_ROUNDS) break;
+                // the status so far (the flips left, and how far the points left their cells)
+                DGT_TRY(cudaMemcpyAsync(c->h_st, dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
+                DGT_TRY(cudaStreamSynchronize(s));
+                skin_known = fold && c->h_st->skin_measured <= MAX_SKIN_CELLS;
+                if (c->h_st->flip_count[fr & 1] <= c->sms * SPILL_EDGES_PER_SM) break;
             }
-            if (fixed_rounds > 0 || fr >= MAX_FLIP_ROUNDS) break;
-            int left = 0;
-            DGT_TRY(cudaMemcpyAsync(&left, &dst->flip_count[fr & 1], sizeof(int), cudaMemcpyDeviceToHost, s));
-            DGT_TRY(cudaStreamSynchronize(s));
-            if (left <= c->sms * SPILL_EDGES_PER_SM) break;
+            f.cur = flips[fr & 1];
+            f.cur_count = counts[fr & 1];
+            c->launches += 1;
+            DGT_TRY(launch_flip_spill(f, fr, ctl, max_skin, c->sms, s));
         }
-        f.cur = flips[fr & 1];
-        f.cur_count = &dst->flip_count[fr & 1];
-        c->launches += 2;
-        DGT_TRY(launch_flip_spill(f, fr, ctl, c->sms, s));
     }
-    if (fold) {
-        // timed as the bin phase (inside the repair phase's span)
+    if (fold && !skin_known) {
+        // (known: the host has seen that the cell lists stay.)  Timed as the bin phase, inside
+        // the repair phase's span
         PhaseTimer bt(c, DGT_PHASE_BIN, s);
-        DGT_TRY(launch_rebin_decide(dst, MAX_SKIN_CELLS, s));
         BinArgs a = bin_args(c, d_points);
         a.cond = &dst->rebin;
-        DGT_TRY(launch_clear_counts(c->ccount.as<int>(), c->total_cells + 1, c->bcount.as<int>(), c->total_blocks + 1,
-                                    a.cond, s));
-        DGT_TRY(launch_bin_st(a, dst, s));
-        c->launches += 2 + (c->n > 0 ? 3 : 0) + 3 + (c->deterministic && c->total_cells > 0 ? 1 : 0);
+        DGT_TRY(launch_bin_all(a, dst, false, &c->launches, s));
     }
     if (c->flip) {
         c->launches += 1;
@@ -900,7 +900,6 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
                               &ctl->epoch, c->sms, s));
     }
     int round = 0;
-    bool pending = false;
     for (;;) {
         // a batch of rounds; each kernel reads its item count on the device
         int batch = fixed_rounds > 0 ? fixed_rounds : (round == 0 ? FIRST_ROUNDS : NEXT_ROUNDS);
@@ -925,20 +924,19 @@ int repair_impl(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, i
             DGT_TRY(run_rings(c, a, s));
         }
         if (fixed_rounds > 0) break;
-        int left = 0;
-        DGT_TRY(cudaMemcpyAsync(&left, list_counts[round & 1], sizeof(int), cudaMemcpyDeviceToHost, s));
+        // the end of the call, unless points are left in the list
+        phase_end(c, DGT_PHASE_REPAIR, s);
+        c->launches += 1;
+        DGT_TRY(launch_call_end(ctl, dst, round, s, md != nullptr, true, c->h_st));
         DGT_TRY(cudaStreamSynchronize(s));
-        if (left == 0) break;
-        if (round > 256) {
-            pending = true;
-            break;
-        }
+        if ((round & 1 ? c->h_st->list_count1 : c->h_st->list_count0) == 0) return conclude(c, s, false);
+        if (round > 256) break;
     }
     phase_end(c, DGT_PHASE_REPAIR, s);
     c->launches += 1;
-    DGT_TRY(launch_call_end(ctl, dst, round, s, md != nullptr));
+    DGT_TRY(launch_call_end(ctl, dst, round, s, md != nullptr, false, conclude_now ? c->h_st : nullptr));
     if (!conclude_now) return DGT_OK;
-    return conclude(c, s, pending);
+    return conclude(c, s, fixed_rounds == 0);
 }
 
 }  // namespace
@@ -1401,7 +1399,6 @@ int dgt_autotune(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, 
     set_relative_cell(c, 1.0);
     int r = init_context(c);
     if (r != DGT_OK) return r;
-    DGT_TRY(cudaMemsetAsync(c->st.p, 0, sizeof(DevStatus), s));
     DGT_TRY(run_bin(c, d_points, s));
     int *dmax = &c->st.as<DevStatus>()->need_stride;   // scratch word: every call clears the status
     DGT_TRY(cudaMemsetAsync(dmax, 0, sizeof(int), s));

@@ -321,7 +321,10 @@ cudaError_t launch_bin_st(const BinArgs &a, DevStatus *st, cudaStream_t s);
 // a.cond = &st->rebin then runs only when needed, all decided on the device.
 cudaError_t launch_refresh(const BinArgs &a, DevStatus *st, float max_skin, cudaStream_t s);
 cudaError_t launch_rebin_decide(DevStatus *st, float max_skin, cudaStream_t s);
-cudaError_t launch_clear_counts(int *ccount, int ncell, int *bcount, int nblock, const int *cond, cudaStream_t s);
+cudaError_t launch_clear_counts(int *ccount, int ncell, int *bcount, int nblock, DevStatus *st, const int *cond,
+                                cudaStream_t s);
+constexpr int BIN_SMALL_MAX = 4096;    // points that one block bins (k_bin_small)
+cudaError_t launch_bin_all(const BinArgs &a, DevStatus *st, bool clear_status, int *launches, cudaStream_t s);
 constexpr float MAX_SKIN_CELLS = 0.5f;
 cudaError_t launch_scan(const int *in, int n, int *bsum, int *out, cudaStream_t s);
 int scan_block_count(int n);
@@ -385,8 +388,13 @@ cudaError_t launch_validate(const SetDesc *sets, const int *set_of, const double
                             const int *nn, int stride, int n, unsigned long long *out, int sms, int general,
                             cudaStream_t s);
 cudaError_t launch_flip_round(const FlipArgs &a, int round, int sms, cudaStream_t s);
-// leftover candidates to the rebuild list; advances the context's flip stamp by rounds + 1
-cudaError_t launch_flip_spill(const FlipArgs &a, int rounds, DevCtl *ctl, int sms, cudaStream_t s);
+// leftover candidates to the rebuild list; advances the context's flip stamp by rounds + 1;
+// max_skin >= 0: decides whether the cell lists can stay (launch_rebin_decide's decision)
+cudaError_t launch_flip_spill(const FlipArgs &a, int rounds, DevCtl *ctl, float max_skin, int sms, cudaStream_t s);
+// sets of at most FLIP_SMALL_MAX points: up to `rounds` rounds and the spill in one launch
+constexpr int FLIP_SMALL_MAX = 16384;
+cudaError_t launch_flip_small(const FlipArgs &a, int rounds, DevCtl *ctl, int2 *const lists[2], int *const counts[2],
+                              float max_skin, cudaStream_t s);
 cudaError_t launch_restride(const int *src, int old_stride, int *dst, int new_stride, const int *nn, int n,
                             cudaStream_t s);
 // step_ptr != null: the step comes from (and is advanced in) device memory
@@ -400,8 +408,11 @@ cudaError_t launch_displace_md(double2 *pos, int n, const SetDesc *sets, const i
                                unsigned long long seed, unsigned long long *step_ptr, const int *cell_of,
                                DevStatus *st, cudaStream_t s);
 // end of a test-and-repair call: fold flags into the sticky word, check convergence,
-// advance the epoch by rounds + 1 (and the displacement step counter when advance_step)
-cudaError_t launch_call_end(DevCtl *ctl, DevStatus *st, int rounds, cudaStream_t s, bool advance_step = false);
+// advance the epoch by rounds + 1 (and the displacement step counter when advance_step).
+// tentative: only if no point is left in the last round's list.  host_out (pinned): a copy of
+// the status, so that the host needs no copy of its own
+cudaError_t launch_call_end(DevCtl *ctl, DevStatus *st, int rounds, cudaStream_t s, bool advance_step = false,
+                            bool tentative = false, DevStatus *host_out = nullptr);
 // first rebuild round of a flip-mode repair: the current ring neighbours of its points join it
 cudaError_t launch_expand(int *list, int *count, int cap, const int *tri, const int *nn, int stride, int n,
                           int *mark, const int *epoch_ptr, int sms, cudaStream_t s);

@@ -430,6 +430,7 @@ __global__ void __launch_bounds__(WARP_KERNEL_WARPS * 32, 2) k_build_warp(RingAr
     const bool direct = A.worklist && item_count(A) <= A.warp_items;
     const int n = direct ? item_count(A) : min(*A.defer_count, A.npoints);
     const int *list = direct ? A.worklist : A.defer_list;
+    if ((int)blockIdx.x * WARP_KERNEL_WARPS >= n) return;   // (usually all of them)
     for (int item = blockIdx.x * WARP_KERNEL_WARPS + wib; item < n; item += gridDim.x * WARP_KERNEL_WARPS) {
         const int e = list[item];
         const int pid = e < 0 ? ~e : e;
@@ -882,24 +883,35 @@ cudaError_t launch_expand(int *list, int *count, int cap, const int *tri, const 
     return cudaGetLastError();
 }
 
-__global__ void k_call_end(DevCtl *ctl, DevStatus *st, int rounds, int advance_step)
+__global__ void __launch_bounds__(128) k_call_end(DevCtl *ctl, DevStatus *st, int rounds, int advance_step, int tentative,
+                                                  DevStatus *host_out)
 {
-    if (advance_step) ctl->step += 1;
-    int f = st->err_flags;
-    if (rounds > 0) {
-        if ((rounds & 1 ? st->list_count1 : st->list_count0) > 0) {
-            f |= EF_NOT_CONVERGED;
-            st->err_flags |= EF_NOT_CONVERGED;
+    if (threadIdx.x == 0) {
+        const int left = rounds > 0 ? (rounds & 1 ? st->list_count1 : st->list_count0) : 0;
+        if (!(tentative && left > 0)) {
+            if (advance_step) ctl->step += 1;
+            int f = st->err_flags;
+            if (rounds > 0) {
+                if (left > 0) {
+                    f |= EF_NOT_CONVERGED;
+                    st->err_flags |= EF_NOT_CONVERGED;
+                }
+                ctl->epoch += rounds + 1;
+                ctl->calls += 1;
+            }
+            ctl->sticky |= f;
         }
-        ctl->epoch += rounds + 1;
-        ctl->calls += 1;
     }
-    ctl->sticky |= f;
+    __syncthreads();
+    if (host_out)
+        for (int k = threadIdx.x; k < (int)(sizeof(DevStatus) / sizeof(int)); k += blockDim.x)
+            reinterpret_cast<volatile int *>(host_out)[k] = reinterpret_cast<const volatile int *>(st)[k];
 }
 
-cudaError_t launch_call_end(DevCtl *ctl, DevStatus *st, int rounds, cudaStream_t s, bool advance_step)
+cudaError_t launch_call_end(DevCtl *ctl, DevStatus *st, int rounds, cudaStream_t s, bool advance_step, bool tentative,
+                            DevStatus *host_out)
 {
-    k_call_end<<<1, 1, 0, s>>>(ctl, st, rounds, advance_step ? 1 : 0);
+    k_call_end<<<1, 128, 0, s>>>(ctl, st, rounds, advance_step ? 1 : 0, tentative ? 1 : 0, host_out);
     return cudaGetLastError();
 }
 

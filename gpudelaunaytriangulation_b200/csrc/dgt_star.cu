@@ -712,6 +712,7 @@ __global__ void __launch_bounds__(SMALL ? 128 : STAR_BLOCK) k_star(RingArgs A)
         atomicMax(&A.st->rounds, A.round + 1);
     }
     if (IDX && n <= A.wrap_items) return;   // a short list: k_wrap takes it
+    if ((int)blockIdx.x * B >= n) return;
     for (int base = blockIdx.x * B; base < n; base += gridDim.x * B) {
         const int it = base + t;
         const bool act = it < n;

@@ -534,6 +534,11 @@ __global__ void __launch_bounds__(WRAP_WARPS * 32) k_wrap(RingArgs A)
     int maxr = 0;
     const bool handed = A.wrap_mode == WRAP_HANDED || (A.wrap_mode == WRAP_REPAIR && item_count(A) > A.wrap_items);
     const int n = handed ? min(*A.star_count, A.n_items) : item_count(A);
+    if (A.count_round && blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
+        atomicAdd(&A.st->repaired, (unsigned long long)n);
+        atomicMax(&A.st->rounds, A.round + 1);
+    }
+    if ((int)blockIdx.x * WRAP_WARPS >= n) return;
     for (int item = blockIdx.x * WRAP_WARPS + wib; item < n; item += gridDim.x * WRAP_WARPS) {
         int pid, slot = 0;
         bool over = false;

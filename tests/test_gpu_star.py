@@ -107,3 +107,32 @@ def test_rebuild_rounds(n, sigma):
     L = float(np.sqrt(n))
     pts = W.uniform_points(n, L, 95)
     _same(pts, (L, L), 1.0, moved=W.displace(pts, sigma, L, L, 96))
+
+
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 16_384, 16_385])
+def test_small_set_kernels(n):
+    # the one-block binning and flips on either side of the sizes they are taken for: the same
+    # cell order and triangulations as the launches of a large set (a batch with an empty
+    # large set beside it goes the other way)
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayBatch, DelaunayGPU
+
+    L = float(np.sqrt(n))
+    pts = W.uniform_points(n, L, 700 + n)
+    moved = W.displace(pts, 0.05, L, L, 701)
+    big = W.uniform_points(20_000, 200.0, 702)
+    one = DelaunayGPU(n, 20, 1.0, (L, L))
+    two = DelaunayBatch([n, 20_000], [(L, L), (200.0, 200.0)], 20, 1.0)
+    P1 = torch.from_numpy(pts).cuda()
+    P2 = torch.from_numpy(np.concatenate([pts, big])).cuda()
+    t1, k1 = one.globalDelaunayTriangulation(P1)
+    t2, k2 = two.globalDelaunayTriangulation(P2)
+    assert torch.equal(k1, k2[:n]) and torch.equal(t1, t2[: t1.numel()])
+    assert torch.equal(one.cellOrder(), two.cellOrder()[:n])
+    P1.copy_(torch.from_numpy(moved))
+    P2[:n].copy_(P1)
+    one.testAndRepairDelaunayTriangulation(P1, t1, k1)
+    two.testAndRepairDelaunayTriangulation(P2, t2, k2)
+    rows = torch.arange(20, device="cuda")[None, :] < k1[:, None]
+    assert torch.equal(k1, k2[:n]) and torch.equal(t1.view(n, -1)[rows], t2[: t1.numel()].view(n, -1)[rows])
+    assert one.validate(P1, t1, k1)["valid"] == 1
+    assert one.stats()["flips"] > 0
