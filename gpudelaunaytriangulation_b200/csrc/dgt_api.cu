@@ -64,10 +64,11 @@ constexpr int SPILL_EDGES_PER_SM = 64;
 // Work lists of at most this many points per SM go to the warp-per-point kernel whole (two
 // points per resident warp)
 constexpr int WARP_ITEMS_PER_SM = 16;
-// Up to this many points a warp per point throughout: 10,000 points build in 54 us, with a thread
-// per point first in 69 + 66 + 28 us; 45,000 points of a rebuild round in 342 us against 160 + 50 us
-constexpr int WRAP_BUILD_MAX = 20000;
-constexpr int WRAP_REPAIR_MAX = 20000;
+// Up to this many points a warp per point throughout (at 20,000 / 40,000 / 64,000: a build of 30,000
+// points 160 / 144 / 145 us, of 50,000 points 165 / 165 / 196 us; the 4M repair, whose rounds hold
+// 27,000 and 32,000 points, 1548 / 1506 / 1500 us, the 1M one with 45,000 and 59,000 882 / 885 / 981)
+constexpr int WRAP_BUILD_MAX = 40000;
+constexpr int WRAP_REPAIR_MAX = 40000;
 constexpr int MAX_DEFER_CHUNKS = 8;   // slot chunks of an overlapped global build (dgt_set_deferred_overlap)
 constexpr int MAX_FLIP_ROUNDS = 24; // flip rounds of a checked call before the rest is rebuilt
 constexpr int ASYNC_FLIP_ROUNDS = 3; // default flip rounds of an unsynchronised call (best of 1-10 for MD steps at sigma 0.01)

@@ -15,10 +15,10 @@
 //   4. certify: every circle of the ring lies inside the window (and inside the radius the
 //      candidates were cut at), so no point outside it can change the ring; if not, one more
 //      pass over the cells the circles reach, with the candidates that lie in some circle.
-// What bounds it: instruction issue (59% of the issue slots at 16 warps per SM, 22 of 32 lanes
-// active; the incremental kernel has 53% and 10 lanes, and three times the instructions).  4M
-// uniform points: 5.79 ms in the incremental kernel, 1.68 + 0.52 ms in these two launches; 1M
-// lattice sites 0.56 -> 0.28 ms; 1M points with float64 predicates 2.75 -> 1.09 ms.
+// What bounds it: instruction issue (67% of the issue slots at 20 warps per SM, 22 of 32 lanes
+// active; the incremental kernel has 53% and 10 lanes, and several times the instructions).  4M
+// uniform points: 5.79 ms in the incremental kernel, 1.28 + 0.49 ms in these two launches; 1M
+// lattice sites 0.56 -> 0.23 ms; 1M points with float64 predicates 2.75 -> 0.67 + 0.26 ms.
 //
 // Every decision is certain or the point is handed on: a turn the filter cannot decide is
 // re-evaluated with the float64 in-circle predicate; angles closer than their rounding errors

@@ -15,8 +15,8 @@
 //
 // What bounds it: the latency of one point's chain (some 2000 instructions, a few microseconds,
 // against 95 us for a point of the incremental thread-per-point kernel) while the points fit the
-// chip at once, instruction issue beyond.  1,000 points: 22 us against 96 us; 10,000: 54 us against
-// 117 us; the 18k points that the first stage leaves of 4M uniform ones: 134 us.
+// chip at once, instruction issue beyond (53% of the issue slots at 10,000 points).  1,000 points:
+// 20 us against 96 us; 10,000: 42 us against 117 us.
 #include "dgt_star.cuh"
 
 namespace dgt {
@@ -41,6 +41,7 @@ template <typename T> struct WrapMem {
     float2 w[32];          // circles of the ring (2 x centre)
     float d[32];           // their diameters, rounded up
     unsigned char ring[32];
+    int row[32];           // per non-empty range of the rows at hand: first slot less its place in the sequence
 };
 
 // floats ordered as unsigned integers
@@ -118,6 +119,7 @@ struct Wrap {
         const int per = seam ? 16 : 32;   // rows a turn: a row over the edge has two parts
         const bool tight = !GEN && filter && y1 - y0 >= 8;
         const int known = n;
+        bool odd = false;
         for (int r0 = y0; r0 <= y1; r0 += per) {
             const int row = r0 + (seam ? lane >> 1 : lane);
             int start = 0, cnt = 0;
@@ -153,27 +155,42 @@ struct Wrap {
             cand += (unsigned)total;
             if (total > most) return false;
             most -= total;
+            // candidate j of the sequence belongs to the last non-empty range that begins at or before
+            // it: the ranges' offsets in a table, the beginnings within 32 candidates as bits
+            const unsigned filled = __ballot_sync(FULL, cnt > 0);
+            __syncwarp();
+            if (cnt > 0) M.row[__popc(filled & ((1u << lane) - 1u))] = start - excl;
+            __syncwarp();
             for (int base = 0; base < total; base += 32) {
-                const int j = base + lane;
-                int o = 0;   // the last lane whose range starts at or before j
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int e = __shfl_sync(FULL, excl, o + step);
-                    if (e <= j) o += step;
-                }
-                int id = __shfl_sync(FULL, start, o) + j - __shfl_sync(FULL, excl, o);
+                const int j = base + lane, at0 = excl - base;
+                const unsigned begins = __reduce_or_sync(FULL, cnt > 0 && (unsigned)at0 < 32u ? 1u << at0 : 0u);
+                const int before = base == 0 ? 0 : __popc(__ballot_sync(FULL, cnt > 0 && at0 < 0));
+                const int rank = before - 1 + __popc(begins & (FULL >> (31 - lane)));
+                int id = M.row[rank] + j;
                 bool keep = j < total;
                 T dx = (T)0, dy = (T)0, nd = (T)1;
                 if (keep) {
                     if (IDX) id = __ldg(&A.sidx[id]);
                     const double2 c = __ldg(IDX ? &A.pos[id] : &A.spos[id]);
-                    const double2 d = GEN ? gen_off(c, p, S) : make_double2(wrap_off(c.x, p.x, S.Lx, S.hLx),
-                                                                           wrap_off(c.y, p.y, S.Ly, S.hLy));
+                    double2 d;
+                    if (GEN) {
+                        d = gen_off(c, p, S);
+                    } else {
+                        // (wrap_off with one comparison in the common case)
+                        d = make_double2(__dsub_rn(c.x, p.x), __dsub_rn(c.y, p.y));
+                        if (fabs(d.x) > S.hLx) d.x = wrap_off(c.x, p.x, S.Lx, S.hLx);
+                        if (fabs(d.y) > S.hLy) d.y = wrap_off(c.y, p.y, S.Ly, S.hLy);
+                    }
                     dx = PR::from64(d.x);
                     dy = PR::from64(d.y);
                     nd = dx * dx + dy * dy;
-                    keep = id != self && !(d.x == 0.0 && d.y == 0.0) && nd <= r2;
-                    // (a safe range for squares and reciprocals; outside it nothing is certain here)
-                    if (keep && !(nd > (T)1e-30 && nd < (T)1e30)) n = WRAP_CAP + 1;
+                    keep = id != self && nd <= r2;
+                    // outside the safe range of squares and reciprocals nothing is certain here
+                    // (except that a coincident point is no neighbour)
+                    if (keep && !(nd > (T)1e-30 && nd < (T)1e30)) {
+                        odd |= d.x != 0.0 || d.y != 0.0;
+                        keep = false;
+                    }
                 }
                 if (filter && keep) {
                     const T l1 = fabs(dx) + fabs(dy);
@@ -185,10 +202,6 @@ struct Wrap {
                 }
                 if (keep)
                     for (int k = 0; k < known; ++k) keep &= M.id[k] != id;
-                if (__any_sync(FULL, n > WRAP_CAP)) {
-                    n = WRAP_CAP + 1;
-                    return false;
-                }
                 const unsigned got = __ballot_sync(FULL, keep);
                 if (got) {
                     const int at = n + __popc(got & ((1u << lane) - 1u));
@@ -199,12 +212,13 @@ struct Wrap {
                     }
                     n += __popc(got);
                     if (n > WRAP_CAP) {
-                        n = WRAP_CAP;
+                        n = __any_sync(FULL, odd) ? WRAP_CAP + 1 : WRAP_CAP;
                         return false;
                     }
                 }
             }
         }
+        if (__any_sync(FULL, odd)) n = WRAP_CAP + 1;
         return true;
     }
 
@@ -214,15 +228,18 @@ struct Wrap {
         return star_recheck<GEN, true>(IDX ? A.pos : A.spos, &S, p, M.id[ka], M.id[kb], M.id[kc]);
     }
 
-    // the hull of the n candidates: M.ring[0 .. m).  1: done, 0: open, -1: not decided here
+    // the hull of the n <= 32 K candidates: M.ring[0 .. m).  1: done, 0: open, -1: not decided
+    // here.  (A form for two candidates a lane and one for four: with the places beyond n skipped
+    // at run time 10,000 points took 50 us, the compiler predicates them.)
+    template <int K>
     __device__ __forceinline__ int walk()
     {
-        V2 c[WRAP_K];
-        T ec[WRAP_K];
+        V2 c[K];
+        T ec[K];
         unsigned far = 0;
         int first = 0;
 #pragma unroll
-        for (int j = 0; j < WRAP_K; ++j) {
+        for (int j = 0; j < K; ++j) {
             const int k = lane + 32 * j;
             c[j] = k < n ? M.q[k] : PR::mk2((T)0, (T)0);
             ec[j] = err1<T>(c[j]);
@@ -235,42 +252,48 @@ struct Wrap {
         const unsigned most = __reduce_max_sync(FULL, far);
         first = __shfl_sync(FULL, first, __ffs(__ballot_sync(FULL, far == most)) - 1);
         int ka = first;
+        const bool check = A.check != 0;
         m = 0;
         for (int guard = 0; guard < 2 * WRAP_CAP; ++guard) {
             const V2 a = M.q[ka];
             const T ea = err1<T>(a);
             // slope of a' -> c' in the frame (tangent, inward) of a'; only directions within half a
-            // turn ahead
-            unsigned best = FULL;
-            int kb = 0;
+            // turn ahead (not the vertex itself, nor the origin that stands in for places without a
+            // candidate: fused, their tangent parts are rounding errors of either sign)
+            float best = 3e38f;
+            int kb = -1;
+            V2 v[K];
 #pragma unroll
-            for (int j = 0; j < WRAP_K; ++j) {
-                if (32 * j < n) {
-                    const T u = a.x * c[j].y - a.y * c[j].x;
-                    const T v = a.x * (a.x - c[j].x) + a.y * (a.y - c[j].y);
-                    const unsigned key = ordered((float)v * rcp_fast((float)u));
-                    // (not the vertex itself: fused, its own u is a rounding error)
-                    if ((float)u > 0.0f && key < best && lane + 32 * j != ka) {
-                        best = key;
-                        kb = lane + 32 * j;
+            for (int j = 0; j < K; ++j) {
+                {
+                    v[j] = PR::mk2(c[j].x - a.x, c[j].y - a.y);
+                    const float u = (float)(a.x * v[j].y - a.y * v[j].x);
+                    const float slope = -(float)(a.x * v[j].x + a.y * v[j].y) * rcp_fast(u);
+                    const int k = lane + 32 * j;
+                    if (u > 0.0f && slope < best && k != ka && k < n) {
+                        best = slope;
+                        kb = k;
                     }
                 }
             }
-            const unsigned least = __reduce_min_sync(FULL, best);
+            const unsigned key = kb >= 0 ? ordered(best) : FULL, least = __reduce_min_sync(FULL, key);
             if (least == FULL) return 0;
-            kb = __shfl_sync(FULL, kb, __ffs(__ballot_sync(FULL, best == least)) - 1);
+            const unsigned who = __ballot_sync(FULL, key == least);
+            kb = __shfl_sync(FULL, kb, __ffs(who) - 1);
             // every other candidate to the left of the edge
             for (;;) {
                 const V2 b = M.q[kb];
-                const T eb = err1<T>(b);
+                const T eb = err1<T>(b), ux = b.x - a.x, uy = b.y - a.y;
+                const T lu = fabs(ux) + fabs(uy), eab = ea + eb;
                 unsigned open = 0;
 #pragma unroll
-                for (int j = 0; j < WRAP_K; ++j) {
-                    if (32 * j < n) {
+                for (int j = 0; j < K; ++j) {
+                    {
+                        // (turn() with the differences at hand)
                         const int k = lane + 32 * j;
-                        T o, bnd;
-                        turn<T>(a, b, c[j], ea, eb, ec[j], o, bnd);
-                        open |= (unsigned)(k < n && k != ka && k != kb && (!(o > bnd) || A.check)) << j;
+                        const T o = ux * v[j].y - uy * v[j].x;
+                        const T bnd = (fabs(v[j].x) + fabs(v[j].y)) * eab + (lu * (ea + ec[j]) + PR::tiny());
+                        open |= (unsigned)(k < n && k != ka && k != kb && (!(o > bnd) || check)) << j;
                     }
                 }
                 ++tests;
@@ -361,7 +384,7 @@ struct Wrap {
             __syncwarp();
             int r;
             for (bool corners = false;; corners = true) {
-                r = n >= 3 ? walk() : 0;
+                r = n < 3 ? 0 : (n <= 64 ? walk<2>() : walk<WRAP_K>());
                 if (r != 0 || corners) break;
                 // open: with the virtual corners
                 if (n + 4 > WRAP_CAP || !first) return W_FAIL;
