@@ -28,9 +28,13 @@ constexpr int WRAP_K = WRAP_CAP / 32;
 constexpr int WRAP_WARPS = 4;      // points per block
 constexpr int WRAP_PASSES = 64;
 constexpr float WRAP_TARGET = 50.0f;   // candidates a first window is sized for
-// candidates a point may scan before the incremental warp kernel takes it (rims of dense clusters:
-// that kernel skips empty space by occupancy blocks and scans nearest tiles first; 1M points in 64
-// clusters, three seeds: 7.7-10.7 ms at 1024, 6.4-9.6 at 4096, 3.9-7.6 at 16384, 5.6-8.5 at 32768)
+// Points whose circles reach over more cells per axis, or that scan more candidates, go to the
+// incremental warp kernel, which skips empty space by occupancy blocks and scans nearest tiles
+// first (points in the voids between dense clusters, and on their rims).  Geometric mean over
+// twelve clustered sets of 0.25 to 1M points: 3.29 / 3.17 / 3.24 / 3.53 / 3.69 ms at 48 / 70 / 100 /
+// 300 / 900 cells, 4.77 without the first limit; at 70 cells and 8,192 / 16,384 / 32,768 candidates
+// 3.50 / 3.17 / 3.18 ms.
+constexpr int WRAP_REACH = 71;
 constexpr unsigned WRAP_WORK = 16384;
 constexpr unsigned FULL = 0xffffffffu;
 
@@ -472,6 +476,7 @@ struct Wrap {
             grow(y0, y1, b0, b1, ey, S.ysize, gy0, gy1);
             // (unbounded in the whole box)
             if (!all_good && gx0 == x0 && gx1 == x1 && gy0 == y0 && gy1 == y1) return W_FAIL;
+            if (gx1 - gx0 >= WRAP_REACH || gy1 - gy0 >= WRAP_REACH) return W_FAIL;
             x0 = gx0, x1 = gx1, y0 = gy0, y1 = gy1;
             // the ring to the front, its circles beside it
             __syncwarp();
