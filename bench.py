@@ -43,16 +43,16 @@ WORKLOADS = {
     "build_repair_1m": (1_000_000, 1000.0, 0.02, 1.0, 16),
 }
 
-# Algorithmic (compulsory) DRAM bytes per point of the one-ring kernel k_build: own position
+# Algorithmic (compulsory) DRAM bytes per point of the one-ring construction: own position
 # (16 B) + own index (4 B) + cell start (4 B) + ring written (6 neighbours x 4 B on average,
 # exactly 6 on the torus) + ring length (4 B).  Candidate re-reads served on chip are not
 # counted.
 BUILD_BYTES_PER_POINT = 16 + 4 + 4 + 24 + 4
-# DRAM bytes per point that ncu measured for k_build (dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch / points) on a 1,048,576-point capture of the same
+# DRAM bytes per point that ncu measured for the one-ring kernels (k_star twice and k_wrap:
+# dram__bytes_read.sum + dram__bytes_write.sum of the three launches / points) on a 1,048,576-point capture of the same
 # kernel (the --profile build case below); traffic scales with the number of points at fixed
 # density, so the 4M launch is reported as this figure times its points.
-BUILD_DRAM_BYTES_PER_POINT_NCU = 87.3
+BUILD_DRAM_BYTES_PER_POINT_NCU = 164.3
 FALLBACK_HBM_GBS = 6650.0
 
 
@@ -652,7 +652,7 @@ def run_ours(args):
                    "l2": "working set (positions 64 MB x2 + rings 268 MB) larger than the 126 MB L2",
                    "parallelism": f"{world} independent replica(s)"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": traffic, "kernel": "k_build<float,14,64> (one-ring construction)",
+                     "traffic": traffic, "kernel": "k_star (two launches) + k_wrap (one-ring construction)",
                      "bytes_per_point": BUILD_BYTES_PER_POINT, "avg_launch_ms": avg_build_s * 1e3,
                      "peak_source": f"{peak_kind} hbm_gbs"},
         "cpu_baseline": cpu,

@@ -434,12 +434,6 @@ cudaError_t launch_refresh(const BinArgs &a, DevStatus *st, float max_skin, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_rebin_decide(DevStatus *st, float max_skin, cudaStream_t s)
-{
-    k_rebin_decide<<<1, 1, 0, s>>>(st, max_skin);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_clear_counts(int *ccount, int ncell, int *bcount, int nblock, DevStatus *st, const int *cond,
                                 cudaStream_t s)
 {

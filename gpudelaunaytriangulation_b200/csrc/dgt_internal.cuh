@@ -316,11 +316,10 @@ cudaError_t launch_bin_st(const BinArgs &a, DevStatus *st, cudaStream_t s);
 // Repair without a full rebin.  The cell lists of the last binning stay usable as candidate
 // lists while no point lies more than MAX_SKIN_CELLS cells outside the cell that lists it:
 // launch_refresh copies the current positions into cell order and measures that distance
-// (st->skin_measured, in cells), launch_rebin_decide sets st->rebin (too far) and st->skin
+// (st->skin_measured, in cells), and sets st->rebin (too far) and st->skin
 // (the margin the ring kernels must add; 0 after a rebin); binning launched with
 // a.cond = &st->rebin then runs only when needed, all decided on the device.
 cudaError_t launch_refresh(const BinArgs &a, DevStatus *st, float max_skin, cudaStream_t s);
-cudaError_t launch_rebin_decide(DevStatus *st, float max_skin, cudaStream_t s);
 cudaError_t launch_clear_counts(int *ccount, int ncell, int *bcount, int nblock, DevStatus *st, const int *cond,
                                 cudaStream_t s);
 constexpr int BIN_SMALL_MAX = 4096;    // points that one block bins (k_bin_small)
@@ -389,7 +388,7 @@ cudaError_t launch_validate(const SetDesc *sets, const int *set_of, const double
                             cudaStream_t s);
 cudaError_t launch_flip_round(const FlipArgs &a, int round, int sms, cudaStream_t s);
 // leftover candidates to the rebuild list; advances the context's flip stamp by rounds + 1;
-// max_skin >= 0: decides whether the cell lists can stay (launch_rebin_decide's decision)
+// max_skin >= 0: decides whether the cell lists can stay (launch_refresh's decision)
 cudaError_t launch_flip_spill(const FlipArgs &a, int rounds, DevCtl *ctl, float max_skin, int sms, cudaStream_t s);
 // sets of at most FLIP_SMALL_MAX points: up to `rounds` rounds and the spill in one launch
 constexpr int FLIP_SMALL_MAX = 16384;

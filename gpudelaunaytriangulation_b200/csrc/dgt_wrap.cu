@@ -343,6 +343,8 @@ struct Wrap {
         return -1;
     }
 
+    // (A window of three cells may scan WRAP_WORK candidates: dense cells, as of a clustered set at the
+    // mean spacing, 5,850 a point: 1M points 62 ms in the incremental kernels, 37 ms here.)
     // the whole construction; W_OK: lane k < m holds the ring's k-th entry in `out`
     __device__ __forceinline__ int run(int &out)
     {
@@ -370,13 +372,14 @@ struct Wrap {
             // what is there already: nothing, or the ring
             n = first ? 0 : m;
             const unsigned seen = cand;
-            const bool fits = gather(x0, x1, y0, y1, r2, filter, first ? 8 * WRAP_CAP : (int)WRAP_WORK);
+            const bool fits = gather(x0, x1, y0, y1, r2, filter, first && W > 3 ? 8 * WRAP_CAP : (int)WRAP_WORK);
             if (n > WRAP_CAP || cand > WRAP_WORK) return W_FAIL;
             if (first && !fits) {
                 // denser here: the smallest window that holds a disc of WRAP_TARGET candidates at the
                 // local density, cut to that disc; then half as many
                 if (r2 == PR::inf()) r2 = (T)(WRAP_TARGET * (float)(W * W) / (3.14159265f * (float)(cand - seen))) * cell_area;
                 else r2 *= (T)0.5;
+                if (W == 3 && cand - seen > WRAP_WORK) return W_FAIL;
                 const float reach = sqrtf((float)(r2 / cell_area));   // in cells
                 W = min(W, max(3, (int)ceilf(1.0f + 2.0f * reach)));
                 window();

@@ -241,14 +241,16 @@ int dgt_clear_flags(dgt_context *ctx, void *stream);
 /* Kernel shape of the one-ring kernel: (ring entries kept on chip, threads per block) =
  * 0: (14, 64) default, 1: (12, 64), 2: (16, 64), 3: (14, 32), 4: (12, 32), one thread per
  * point; 5: (14, 64) with a group of 4 lanes per point, 6: (14, 64) with 8 lanes per point.
- * Rings longer than the on-chip capacity continue on the deferred (warp-per-point) path, so
- * every shape gives the same output.  The shape applies to global triangulations; the
+ * Shapes 0 to 4 are those of the incremental kernel, which runs only with a work budget below
+ * 256: otherwise the hull kernels take the points first and the warp-per-point kernel what they
+ * leave.  Shapes 5 and 6 replace both.  Every shape gives the same output.  The shape applies to global triangulations; the
  * rebuild rounds of test-and-repair always take shape 0. */
 int dgt_set_kernel_shape(dgt_context *ctx, int shape);
 /* Work budget (no reference counterpart): cells plus candidates one point may scan in the
  * thread-per-point kernel before it is handed to the warp-per-point kernel (points on the rim
- * of dense clusters, whose circles reach over large regions).  Default 1024; 0 sends every
- * point to the warp-per-point kernel.  Both kernels give the same rings. */
+ * of dense clusters, whose circles reach over large regions).  Default 1024.  A budget below 256
+ * also leaves out the hull kernels that otherwise come first (their scans may exceed it); 0 sends
+ * every point to the warp-per-point kernel.  All kernels give the same rings. */
 int dgt_set_work_budget(dgt_context *ctx, int budget);
 /* Global triangulations in `chunks` (1-8) pieces of the cell order, the points each piece
  * defers to the warp-per-point kernel rebuilt on a stream of their own while the next pieces
