@@ -99,7 +99,8 @@ __device__ __forceinline__ int *second_ring(const RingArgs &A, int k)
 
 // Shared memory of a block, a column per thread.  SMALL (first pass with the float32 filter):
 // slots as 16-bit offsets from the point's own slot, so that 20 warps fit an SM instead of 16 (4M
-// uniform points: 1.49 -> 1.33 ms); for sets whose windows span fewer than 32,768 slots.
+// uniform points: 1.49 -> 1.33 ms).  Taken when windows span at most 16,000 slots at the sets' mean
+// densities; a point with a range further off than 16 bits reach is handed on (add_seg).
 template <typename T, bool SMALL> struct StarMem {
     typedef typename Prec<T>::T2 V2;
     static constexpr int B = SMALL ? 128 : STAR_BLOCK;
@@ -229,9 +230,13 @@ struct Star {
             return;
         }
         if (SMALL) {
-            // the offsets from the own slot must fit 16 bits (around the set: a window over its seam)
-            const int d = abs(s - self), e = min(d, S.n - d);
-            if (e + c > 32767) {
+            // The offsets from the own slot must fit 16 bits as gather() takes them: the nearest way
+            // round the set's slots if the warp wraps, as it does where this window crosses the
+            // box's edge, else the plain difference (over half of the set where most points lie in
+            // a few rows).  (The nearest way in every gather: 4M uniform points 2.12 -> 2.17 ms; the
+            // edge looked at first: 1M lattice sites 308 -> 314 us.)
+            const int d = abs(s - self);
+            if (d + c > 32767 && (min(d, S.n - d) + c > 32767 || (ocy + y0 >= 0 && ocy + y1 < S.ysize))) {
                 nseg = STAR_SEGS + 1;
                 return;
             }

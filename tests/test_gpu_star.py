@@ -136,3 +136,51 @@ def test_small_set_kernels(n):
     assert torch.equal(k1, k2[:n]) and torch.equal(t1.view(n, -1)[rows], t2[: t1.numel()].view(n, -1)[rows])
     assert one.validate(P1, t1, k1)["valid"] == 1
     assert one.stats()["flips"] > 0
+
+
+# Sets of more than 40,000 points: up to that many a warp per point (k_wrap) takes a build whole,
+# and k_star none of it.
+def _build_big(pts, box, cell, incremental, fp64=False, stride=24, check=False):
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayGPU
+
+    d = DelaunayGPU(len(pts), stride, cell, box)
+    d.setPrecision(not fp64)
+    d.setCheckMode(check)
+    if incremental:
+        d.setWorkBudget(255)
+    tri, nn = d.globalDelaunayTriangulation(torch.from_numpy(pts).cuda())
+    st = d.stats()
+    assert st["mismatches"] == 0 and st["error_flags"] & ~32 == 0, st
+    return tri, nn, st
+
+
+def _same_big(*args, **kw):
+    b = _build_big(*args, True, **kw)
+    for check in (False, True):
+        a = _build_big(*args, False, check=check, **kw)
+        # the incremental path builds in one launch, the first stage in two of k_star and k_wrap
+        assert a[2]["launches"] == b[2]["launches"] + 2
+        assert torch.equal(a[1], b[1])
+        assert torch.equal(a[0], b[0])
+
+
+def _uneven_points(n, part, spread, seed):
+    """`part` of n points in one row of unit cells, over its whole length or (spread) normal about
+    its middle, the others uniform; returns (points, L)."""
+    L = float(np.sqrt(n))
+    k = int(part * n)
+    h = L / int(L)
+    pts = W.uniform_points(n, L, seed)
+    pts[:k, 1] = (int(L / 2) + pts[:k, 1] / L) * h
+    if spread:
+        pts[:k, 0] = L / 2 + spread * W.normal_pairs(seed + 1, k)[:, 0]
+    return W.wrap(pts, L, L), L
+
+
+@pytest.mark.parametrize("n,part,spread", [(60_000, 0.56, 0.0), (60_000, 0.7, 0.0), (100_000, 0.7, 0.0),
+                                           (64_000, 0.5625, 6.0)])
+def test_most_points_in_one_row_of_cells(n, part, spread):
+    # neighbouring rows lie more than half the set and more than 32,767 slots apart in the cell
+    # order, in windows that do not cross the box's edge: slots as 16-bit offsets
+    pts, L = _uneven_points(n, part, spread, 1)
+    _same_big(pts, (L, L), 1.0, stride=64)
