@@ -140,17 +140,29 @@ def test_small_set_kernels(n):
 
 # Sets of more than 40,000 points: up to that many a warp per point (k_wrap) takes a build whole,
 # and k_star none of it.
-def _build_big(pts, box, cell, incremental, fp64=False, stride=24, check=False):
-    from gpudelaunaytriangulation_b200.delaunay import DelaunayGPU
+BIG = 45_000
 
-    d = DelaunayGPU(len(pts), stride, cell, box)
+
+def _build_big(pts, box, cell, incremental, fp64=False, sizes=None, moved=None, stride=24, check=False):
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayBatch, DelaunayGPU
+
+    d = DelaunayBatch(sizes, box, stride, cell) if sizes is not None else DelaunayGPU(len(pts), stride, cell, box)
     d.setPrecision(not fp64)
     d.setCheckMode(check)
     if incremental:
         d.setWorkBudget(255)
-    tri, nn = d.globalDelaunayTriangulation(torch.from_numpy(pts).cuda())
+    P = torch.from_numpy(pts).cuda()
+    tri, nn = d.globalDelaunayTriangulation(P)
     st = d.stats()
     assert st["mismatches"] == 0 and st["error_flags"] & ~32 == 0, st
+    if moved is not None:
+        d.setFlipRepair(False)   # every flagged point through the rebuild rounds
+        P.copy_(torch.from_numpy(moved))
+        d.testAndRepairDelaunayTriangulation(P, tri, nn)
+        again = d.stats()
+        assert again["mismatches"] == 0 and again["error_flags"] & ~32 == 0, again
+        assert again["flagged"] > 40_000   # the first round's list is k_star's
+        tri.view(len(pts), -1).masked_fill_(torch.arange(stride, device="cuda") >= nn[:, None], 0)
     return tri, nn, st
 
 
@@ -184,3 +196,73 @@ def test_most_points_in_one_row_of_cells(n, part, spread):
     # order, in windows that do not cross the box's edge: slots as 16-bit offsets
     pts, L = _uneven_points(n, part, spread, 1)
     _same_big(pts, (L, L), 1.0, stride=64)
+
+
+@pytest.mark.parametrize("n", [40_001, 50_000, 131_071])
+@pytest.mark.parametrize("cell", [0.45, 0.8, 1.0, 1.7, 2.6])
+def test_big_uniform_sets(n, cell):
+    L = float(np.sqrt(n))
+    _same_big(W.uniform_points(n, L, 510 + n), (L, L), cell)
+
+
+@pytest.mark.parametrize("aspect", [0.005, 0.04, 0.3, 5.0])
+def test_big_rectangles(aspect):
+    Lx, Ly = float(np.sqrt(BIG * aspect)), float(np.sqrt(BIG / aspect))
+    _same_big(W.uniform_points(BIG, Lx, 78, Ly), (Lx, Ly), 1.0)
+
+
+@pytest.mark.parametrize("jitter", [1e-7, 1e-4, 0.05])
+def test_big_lattices(jitter):
+    # collinear candidates at every angle (triangular), four near-cocircular ones round every
+    # square
+    pts, Lx, Ly = W.triangular_lattice(214, 214, jitter=jitter, seed=8)
+    _same_big(pts, (Lx, Ly), 1.0)
+    pts, L = W.square_lattice(212 * 212, phase=jitter, seed=8)
+    _same_big(pts, (L, L), 1.0)
+
+
+@pytest.mark.parametrize("cell", [0.2, 1.0])
+def test_big_clusters(cell):
+    pts, L = W.gaussian_mixture(60_000, components=12, sigma=3.0, L=260.0, seed=6)
+    for fp64 in (False, True):
+        _same_big(pts, (L, L), cell, fp64=fp64, stride=32)
+
+
+@pytest.mark.parametrize("scale", [1e-9, 1.0, 1e9])
+@pytest.mark.parametrize("fp64", [False, True])
+def test_big_float64_and_units(scale, fp64):
+    L = float(np.sqrt(BIG))
+    pts = W.uniform_points(BIG, L, 191)
+    _same_big(pts * scale, (L * scale, L * scale), scale, fp64=fp64)
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("shift", [0.0, 3.0])
+def test_big_general_box(fp64, shift):
+    m = np.array(HEX).reshape(2, 2) * float(np.sqrt(BIG / (np.sqrt(3.0) / 2.0)))
+    u = W.uniform_points(BIG, 1.0, 192)
+    # (shift: outside the primary cell too)
+    pts = np.ascontiguousarray((u + np.floor(shift * W.uniform_points(BIG, 1.0, 193))) @ m.T)
+    _same_big(pts, tuple(m.reshape(-1)), 1.0, fp64=fp64)
+
+
+def test_big_batch():
+    sizes = np.array([5000, 0, 64, 45_000, 1000, 300], dtype=np.int64)
+    boxes = np.stack([np.sqrt(np.maximum(sizes, 1).astype(np.float64))] * 2, axis=1)
+    pts = np.concatenate([W.uniform_points(int(k), float(L), 650 + i)
+                          for i, (k, L) in enumerate(zip(sizes, boxes[:, 0])) if k > 0])
+    for fp64 in (False, True):
+        _same_big(pts, boxes, 1.0, sizes=sizes, fp64=fp64)
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("sigma", [0.1, 0.3])
+def test_big_rebuild_rounds(fp64, sigma):
+    # lists of more than 40,000 points, with kept (0.1) and new cell lists
+    n = 90_000
+    L = float(np.sqrt(n))
+    pts = W.uniform_points(n, L, 195)
+    _same_big(pts, (L, L), 1.0, moved=W.displace(pts, sigma, L, L, 196), fp64=fp64)
+    m = np.array(HEX).reshape(2, 2) * float(np.sqrt(n / (np.sqrt(3.0) / 2.0)))
+    pts = np.ascontiguousarray(W.uniform_points(n, 1.0, 197) @ m.T)
+    _same_big(pts, tuple(m.reshape(-1)), 1.0, moved=pts + sigma * W.normal_pairs(198, n), fp64=fp64)
