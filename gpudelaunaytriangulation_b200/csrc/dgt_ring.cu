@@ -624,8 +624,8 @@ __device__ __forceinline__ float2 test_off(double2 q, double2 p, const SetDesc &
 // The test in flip mode, index order (rows, ring lengths and owner positions stream; only the
 // neighbour gathers are random): a valid fan (every triangle strictly CCW, winding once) sends
 // its illegal or undecided spokes (i, P_k) with i < P_k to the flip list (the flip stage decides
-// them exactly); an invalid fan, or one with more than TEST_MAX_EDGES such spokes, queues its
-// point for rebuilding.  Also measures how far the points left the cells that list them
+// them exactly); an invalid fan, or one with more than TEST_MAX_EDGES such spokes or one past its
+// 32nd, queues its point for rebuilding.  Also measures how far the points left the cells that list them
 // (A.rcell_of).  What bounds it: instruction issue; the spokes share their products (the cross
 // product of P_k and P_k+1 serves the orientation and two in-circles), the row is read once and
 // the cell distance only computed for points that changed cell.
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(256, 3) k_test_flip(TestArgs A)
                 const int c = __ldg(&A.rcell_of[i]);
                 if (S.cell_base + cy * S.xsize + cx != c) moved = fmaxf(moved, outside_cell<GEN>(S, c, p));
             }
-            bool bad = m < 3 || m > A.stride || m > 32;
+            bool bad = m < 3 || m > A.stride;
             if (!bad) {
                 // The first TEST_ROW entries with vector loads (a row is a cache line of its own for
                 // every lane, so each load of it costs as much as a neighbour's position), then
@@ -701,8 +701,8 @@ __global__ void __launch_bounds__(256, 3) k_test_flip(TestArgs A)
                 float g1 = prev.x * cur.y, g2 = prev.y * cur.x;
                 float gp = g1 - g2, gph = fabsf(g1) + fabsf(g2);   // prev x cur
                 int cross = 0;
-                bool inverted = false;
-                auto spoke = [&](int k, float2 nxt, int rnxt) {
+                bool inverted = false, late = false;   // late: a failing spoke past the bits of `fail`
+                auto spoke = [&](float2 nxt, int rnxt) {
                     const float nd = nxt.x * nxt.x + nxt.y * nxt.y;
                     g1 = cur.x * nxt.y;
                     g2 = cur.y * nxt.x;
@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(256, 3) k_test_flip(TestArgs A)
                     }
                     cross += cur.y < 0.0f && nxt.y >= 0.0f;
                     inverted |= !ccw;
-                    fail |= (unsigned)(!outside && i < rcur) << k;
+                    const bool failing = !outside && i < rcur;
                     prev = cur;
                     cur = nxt;
                     na = nb;
@@ -731,15 +731,18 @@ __global__ void __launch_bounds__(256, 3) k_test_flip(TestArgs A)
                     gph = gnh;
                     rprev = rcur;
                     rcur = rnxt;
+                    return failing;
                 };
 #pragma unroll
                 for (int k = 0; k + 1 < TEST_ROW; ++k)
-                    if (k < m) spoke(k, k + 1 == m ? d[0] : d[k + 1], k + 1 == m ? e[0] : e[k + 1]);
+                    if (k < m) fail |= (unsigned)spoke(k + 1 == m ? d[0] : d[k + 1], k + 1 == m ? e[0] : e[k + 1]) << k;
                 for (int k = TEST_ROW - 1; k < m; ++k) {
                     const int r = k + 1 == m ? e[0] : valid(row[k + 1]);
-                    spoke(k, k + 1 == m ? d[0] : test_off<GEN>(__ldg(&A.pos[r]), p, S), r);
+                    const bool failing = spoke(k + 1 == m ? d[0] : test_off<GEN>(__ldg(&A.pos[r]), p, S), r);
+                    if (k < 32) fail |= (unsigned)failing << k;
+                    else late |= failing;
                 }
-                bad |= cross != 1 || inverted;
+                bad |= cross != 1 || inverted || late;
             }
             rebuild = bad || __popc(fail) > TEST_MAX_EDGES;
             if (rebuild) fail = 0;

@@ -143,3 +143,37 @@ def test_largest_single_set_and_repair():
     d.testAndRepairDelaunayTriangulation(P, tri, nn)
     assert d.stats()["error_flags"] == 0
     assert d.validate(P, tri, nn)["valid"] == 1
+
+
+@pytest.mark.parametrize("deg", [31, 32, 33, 40, 60])
+def test_rings_over_32_entries(deg):
+    # centres with `deg` neighbours each: a valid ring of any length passes the local test as it
+    # is, and one with few spokes out of place, any of them past the 32nd too, is repaired
+    DelaunayGPU, _ = _dg()
+    n, per = 20_000, 6
+    L = float(np.sqrt(n))
+    pts = W.uniform_points(n, L, 4)
+    a = 2.0 * np.pi * (np.arange(deg) + 0.1 * np.sin(7.0 * np.arange(deg))) / deg
+    rim = (2.0 + 0.01 * np.cos(3.0 * a))[:, None] * np.stack([np.cos(a), np.sin(a)], axis=1)
+    for i in range(per):
+        for j in range(per):
+            c = np.array([(i + 0.5) * L / per, (j + 0.5) * L / per])
+            pts = pts[((pts - c) ** 2).sum(1) > 9.0]
+            pts = np.concatenate([pts, c[None, :], c + rim])
+    pts = np.ascontiguousarray(pts)
+    d = DelaunayGPU(len(pts), 64, 1.0, (L, L))
+    P = torch.from_numpy(pts).cuda()
+    tri, nn = d.globalDelaunayTriangulation(P)
+    assert int((nn == deg).sum()) >= per * per
+    before = tri.clone()
+    d.testAndRepairDelaunayTriangulation(P, tri, nn)
+    st = d.stats()
+    assert st["flagged"] == 0 and st["repaired"] == 0 and st["error_flags"] == 0, st
+    assert torch.equal(tri, before)
+    for sigma in (0.005, 0.05):
+        P.copy_(torch.from_numpy(W.displace(pts, sigma, L, L, 41)))
+        d.testAndRepairDelaunayTriangulation(P, tri, nn)
+        fresh, k = DelaunayGPU(len(pts), 64, 1.0, (L, L)).globalDelaunayTriangulation(P)
+        assert torch.equal(nn, k)
+        assert np.array_equal(O.canonical(tri.view(len(pts), -1).cpu().numpy(), nn.cpu().numpy()),
+                              O.canonical(fresh.view(len(pts), -1).cpu().numpy(), k.cpu().numpy()))
