@@ -131,7 +131,7 @@ struct DevStatus {
     // one memset clears the next round's list with the two counters between the lists
     int list_count0;            // repair work lists (ping-pong)
     int defer_count;            // items queued for the warp-per-point kernel
-    int star_count;             // items the first stage handed to the incremental kernels
+    int star_count;             // items the first stage handed to the warp-per-point hull kernel
     int list_count1;
     int flip_count[2];          // flip candidate lists (ping-pong)
     int second_count;           // slots for the first stage's second pass (global builds)
@@ -148,7 +148,7 @@ struct DevStatus {
     unsigned long long flagged;         // points queued by the test kernel
     unsigned long long repaired;        // points rebuilt by repair rounds
     unsigned long long cells;           // grid cells scanned
-    unsigned long long heavy_points;    // deferred because they outgrew the per-thread work budget
+    unsigned long long heavy_points;    // rebuilt by a warp each, their scan over the work budget
     unsigned long long flips;           // test-and-repair: edge flips applied
     unsigned long long flip_spilled;    // flip candidates left after the last flip round
     int flip_rounds;                    // flip rounds run
@@ -234,8 +234,7 @@ struct RingArgs {
     // scans longer than work_budget (cells + candidates)
     int *defer_list;
     int *defer_count;
-    // points the first stage (dgt_star.cu) hands to the incremental kernels, complemented when
-    // their scan was too large for it
+    // points the first stage (dgt_star.cu) hands to the warp-per-point hull kernel (dgt_wrap.cu)
     int *star_list;
     int *star_count;
     // global builds: slots its first pass could not certify, at most second_cap, and their rings,

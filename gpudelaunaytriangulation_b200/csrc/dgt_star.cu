@@ -86,7 +86,7 @@ __device__ __forceinline__ unsigned angle_key(float x, float y)
 // points that the first could not certify)
 enum { STAR_BOTH = 0, STAR_FIRST = 1, STAR_SECOND = 2 };
 
-enum { S_TODO = 0, S_OK = 1, S_FAIL = 2, S_HEAVY = 3 };
+enum { S_TODO = 0, S_OK = 1, S_FAIL = 2 };
 
 // ring of entry k of the second pass's list: its length, then up to STAR_RING - 1 slots
 constexpr int STAR_RING = 16;
@@ -344,7 +344,7 @@ struct Star {
             }
             if (!keep) continue;
             if (n >= cap) {
-                status = S_HEAVY;
+                status = S_FAIL;
                 break;
             }
             const T iv = rcp_fast(nd);
@@ -481,8 +481,8 @@ struct Star {
 
     // The circles of the ring (2 x centre = the pole of the line through a' and b'): S_OK when they
     // all lie inside the window and within |d|^2 <= r2.  Otherwise the window they reach, with
-    // the circles in q[31 - k] and the largest diameter in wmax; S_FAIL / S_HEAVY when some
-    // circle is not bounded (ill-conditioned or open) or that window is too large.  leave: only the
+    // the circles in q[31 - k] and the largest diameter in wmax; S_FAIL when some circle is not
+    // bounded (ill-conditioned or open) or that window is too large.  leave: only the
     // verdict is wanted.
     __device__ __forceinline__ void certify(T r2, T dropped, bool leave, bool again, T &wmax)
     {
@@ -545,7 +545,7 @@ struct Star {
             return;
         }
         if (again || m > STAR_CAP / 2) {
-            status = S_HEAVY;
+            status = S_FAIL;
             return;
         }
         if (SMALL || leave) return;
@@ -554,7 +554,7 @@ struct Star {
         y0 = (int)floor(b0);
         y1 = (int)floor(b1);
         if (x1 - x0 >= S.xsize || y1 - y0 >= S.ysize || x1 - x0 > 63 || y1 - y0 >= STAR_SEGS) {
-            status = S_HEAVY;
+            status = S_FAIL;
             return;
         }
         // the circles to the top of q, by way of the candidate array (as float pairs)
@@ -620,15 +620,14 @@ struct Star {
             }
         }
         cells += (unsigned)(W * W);
-        if (nseg > STAR_SEGS || total > A.work_budget) status = S_HEAVY;
-        else if (total < 4) status = S_FAIL;
+        if (nseg > STAR_SEGS || total > A.work_budget || total < 4) status = S_FAIL;
     }
     // the window of the second pass (set by certify)
     __device__ __forceinline__ void second_window()
     {
         build_segs();
         cells += (unsigned)((x1 - x0 + 1) * (y1 - y0 + 1));
-        if (nseg > STAR_SEGS || total > A.work_budget) status = S_HEAVY;
+        if (nseg > STAR_SEGS || total > A.work_budget) status = S_FAIL;
     }
     // whether an offset from the window may have to go round the box
     __device__ __forceinline__ bool wraps() const
@@ -659,7 +658,7 @@ struct Star {
     }
 
     // Every lane of the warp calls these (votes inside); active: lanes with a point.  Afterwards
-    // status is S_OK, S_FAIL / S_HEAVY, or (first pass only) S_TODO with the ring of the pass
+    // status is S_OK, S_FAIL, or (first pass only) S_TODO with the ring of the pass
     __device__ __forceinline__ void run(int mode, bool active)
     {
         if (!active) status = S_FAIL;
@@ -760,7 +759,7 @@ __global__ void __launch_bounds__(SMALL ? 128 : STAR_BLOCK) k_star(RingArgs A)
                     row[0] = b.m;
                     for (int k = 0; k < b.m; ++k) row[k + 1] = b.slot(b.ord(k));
                 } else {
-                    A.star_list[atomicAdd(A.star_count, 1)] = b.status == S_FAIL ? pid : ~pid;
+                    A.star_list[atomicAdd(A.star_count, 1)] = pid;
                 }
             }
         }

@@ -61,7 +61,8 @@ __device__ __forceinline__ float unordered(unsigned k)
 __device__ __forceinline__ float warp_min(float x) { return unordered(__reduce_min_sync(FULL, ordered(x))); }
 __device__ __forceinline__ float warp_max(float x) { return unordered(__reduce_max_sync(FULL, ordered(x))); }
 
-enum { W_OK = 0, W_FAIL = 1 };
+// W_HEAVY: not done because its scan would be too large here too
+enum { W_OK = 0, W_FAIL = 1, W_HEAVY = 2 };
 
 template <typename T, bool IDX, bool GEN>
 struct Wrap {
@@ -373,13 +374,14 @@ struct Wrap {
             n = first ? 0 : m;
             const unsigned seen = cand;
             const bool fits = gather(x0, x1, y0, y1, r2, filter, first && W > 3 ? 8 * WRAP_CAP : (int)WRAP_WORK);
-            if (n > WRAP_CAP || cand > WRAP_WORK) return W_FAIL;
+            if (n > WRAP_CAP) return W_FAIL;
+            if (cand > WRAP_WORK) return W_HEAVY;
             if (first && !fits) {
                 // denser here: the smallest window that holds a disc of WRAP_TARGET candidates at the
                 // local density, cut to that disc; then half as many
                 if (r2 == PR::inf()) r2 = (T)(WRAP_TARGET * (float)(W * W) / (3.14159265f * (float)(cand - seen))) * cell_area;
                 else r2 *= (T)0.5;
-                if (W == 3 && cand - seen > WRAP_WORK) return W_FAIL;
+                if (W == 3 && cand - seen > WRAP_WORK) return W_HEAVY;
                 const float reach = sqrtf((float)(r2 / cell_area));   // in cells
                 W = min(W, max(3, (int)ceilf(1.0f + 2.0f * reach)));
                 window();
@@ -479,7 +481,7 @@ struct Wrap {
             grow(y0, y1, b0, b1, ey, S.ysize, gy0, gy1);
             // (unbounded in the whole box)
             if (!all_good && gx0 == x0 && gx1 == x1 && gy0 == y0 && gy1 == y1) return W_FAIL;
-            if (gx1 - gx0 >= WRAP_REACH || gy1 - gy0 >= WRAP_REACH) return W_FAIL;
+            if (gx1 - gx0 >= WRAP_REACH || gy1 - gy0 >= WRAP_REACH) return W_HEAVY;
             x0 = gx0, x1 = gx1, y0 = gy0, y1 = gy1;
             // the ring to the front, its circles beside it
             __syncwarp();
@@ -572,11 +574,8 @@ __global__ void __launch_bounds__(WRAP_WARPS * 32) k_wrap(RingArgs A)
     if ((int)blockIdx.x * WRAP_WARPS >= n) return;
     for (int item = blockIdx.x * WRAP_WARPS + wib; item < n; item += gridDim.x * WRAP_WARPS) {
         int pid, slot = 0;
-        bool over = false;
         if (handed || IDX) {
             pid = handed ? A.star_list[item] : A.worklist[item];
-            over = pid < 0;
-            if (over) pid = ~pid;
             if (!IDX) slot = A.slot_of[pid];
         } else {
             slot = A.item_base + item;
@@ -587,6 +586,8 @@ __global__ void __launch_bounds__(WRAP_WARPS * 32) k_wrap(RingArgs A)
         Wrap<T, IDX, GEN> b(A, S, M, lane, p, IDX ? pid : slot);
         int id = -1;
         const int r = b.run(id);
+        // more than a thread may scan (counted; complemented in the deferred list)
+        const bool over = r == W_HEAVY || b.cells + b.cand > (unsigned)A.work_budget;
         if (r == W_OK) {
             ++pts;
             heavy += over;
@@ -610,11 +611,7 @@ __global__ void __launch_bounds__(WRAP_WARPS * 32) k_wrap(RingArgs A)
         ctr.mism += b.mism;
         __syncwarp();
     }
-    if (handed) {
-        if (lane == 0 && pts) atomicAdd(&A.st->exact_points, (unsigned long long)pts);
-        if (lane == 0 && heavy) atomicAdd(&A.st->heavy_points, (unsigned long long)heavy);
-        pts = 0;
-    }
+    if (lane == 0 && heavy) atomicAdd(&A.st->heavy_points, (unsigned long long)heavy);
     flush_counters(A, ctr, lane == 0 ? pts : 0, maxr);
 }
 

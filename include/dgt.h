@@ -38,7 +38,8 @@ typedef struct dgt_context dgt_context;
 
 /* counters of the last triangulation / test-and-repair call */
 typedef struct dgt_stats {
-    long long points;          /* ring constructions (build: n; repair: rebuilt points) */
+    long long points;          /* ring constructions but those of exact_points (together: build: n;
+                                  repair: rebuilt points) */
     long long candidates;      /* candidate points examined */
     long long tests;           /* circle tests evaluated by the filter stage */
     long long fp32_undecided;  /* tests the float32 filter left open (re-run in float64) */
@@ -57,7 +58,8 @@ typedef struct dgt_stats {
     int reserved;
     long long repair_calls;    /* test-and-repair calls completed on the device */
     long long md_step;         /* device step counter used by DGT_STEP_AUTO */
-    long long heavy_points;    /* points rebuilt by the warp-per-point kernel (over the work budget) */
+    long long heavy_points;    /* points rebuilt by a warp each because their scan was too large for a
+                                  thread (over the work budget) */
     long long flips;           /* test-and-repair: edge flips applied */
     long long flip_spilled;    /* test-and-repair: flip candidates handed to the rebuild rounds */
     int flip_rounds;           /* test-and-repair: flip rounds run */

@@ -524,3 +524,20 @@ def test_autotune_result_is_correct_and_cached():
     d2 = _dg()(n, 16, 1.0, (L, L))
     res2 = d2.autotune(P, tri, nn)
     assert res2["from_cache"] == 1 and res2["shape"] == res["shape"]
+
+
+@pytest.mark.parametrize("n", [30_000, 100_000])
+def test_exact_points_are_the_deferred_ones(n):
+    # every point is counted once: under exact_points those the exact warp kernel rebuilt, which a
+    # uniform set hardly has, under points all others, whichever kernel settled them
+    L = float(np.sqrt(n))
+    d = _dg()(n, 16, 1.0, (L, L))
+    d.globalDelaunayTriangulation(torch.from_numpy(W.uniform_points(n, L, 131)).cuda())
+    st = d.stats()
+    assert st["points"] + st["exact_points"] == n, st
+    assert st["exact_points"] <= n // 10_000 and st["heavy_points"] <= n // 10_000, st
+    pts, L = W.square_lattice(2500, phase=0.0)   # all cocircular: the exact kernel's
+    d = _dg()(2500, 16, 1.0, (L, L))
+    d.globalDelaunayTriangulation(torch.from_numpy(pts).cuda())
+    st = d.stats()
+    assert st["points"] + st["exact_points"] == 2500 and st["exact_points"] > 0, st
