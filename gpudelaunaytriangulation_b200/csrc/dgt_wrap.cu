@@ -122,7 +122,9 @@ struct Wrap {
     {
         const bool seam = ocx + x0 < 0 || ocx + x1 >= S.xsize;
         const int per = seam ? 16 : 32;   // rows a turn: a row over the edge has two parts
-        const bool tight = !GEN && filter && y1 - y0 >= 8;
+        // (a window over a whole axis takes every cell: a row or column of it stands for two distances
+        // from the point, the one it is listed at and the nearest, which candidates are taken at)
+        const bool tight = !GEN && filter && y1 - y0 >= 8 && y1 - y0 + 1 < S.ysize && x1 - x0 + 1 < S.xsize;
         const int known = n;
         bool odd = false;
         for (int r0 = y0; r0 <= y1; r0 += per) {

@@ -266,3 +266,29 @@ def test_big_rebuild_rounds(fp64, sigma):
     m = np.array(HEX).reshape(2, 2) * float(np.sqrt(n / (np.sqrt(3.0) / 2.0)))
     pts = np.ascontiguousarray(W.uniform_points(n, 1.0, 197) @ m.T)
     _same_big(pts, tuple(m.reshape(-1)), 1.0, moved=pts + sigma * W.normal_pairs(198, n), fp64=fp64)
+
+
+@pytest.mark.parametrize("width", [4.7, 5.2, 6.2])
+@pytest.mark.parametrize("cell", [0.3, 0.6, 1.0])
+@pytest.mark.parametrize("rebuild", [False, True])
+def test_narrow_boxes(width, cell, rebuild):
+    # circles close to half the box and past it: windows over the whole short axis (where circles
+    # pass half the box, flag 32, the nearest images still give one answer)
+    sizes = np.arange(60, 360)
+    boxes = np.stack([np.full(300, width), sizes / width], axis=1)
+    pts = np.concatenate([W.uniform_points(int(k), width, 800 + i, float(b[1]))
+                          for i, (k, b) in enumerate(zip(sizes, boxes))])
+    assert len(pts) > 40_000
+    low = sizes.cumsum()[150]
+    for part in (slice(0, 150), slice(0, 300)):   # up to 40,000 points and more
+        p = pts[:low - sizes[150]] if part.stop == 150 else pts
+        moved = None
+        if rebuild:
+            L = np.repeat(boxes[part], sizes[part], axis=0)
+            moved = np.mod(p + 0.2 * W.normal_pairs(801, len(p)), L)
+            moved = np.where(moved >= L, 0.0, moved)
+        b = _rings(p, boxes[part], cell, True, sizes=sizes[part], moved=moved)
+        for fp64 in (False, True):
+            a = _rings(p, boxes[part], cell, False, sizes=sizes[part], moved=moved, fp64=fp64)
+            assert torch.equal(a[1], b[1])
+            assert torch.equal(a[0], b[0])
