@@ -489,7 +489,8 @@ cudaError_t run_rings(dgt_context *c, const RingArgs &a, cudaStream_t s, PhaseTi
     c->launches += any + 1;
     if (c->work_budget >= STAR_MIN_BUDGET && kernel_shape_lanes(shape) == 1) {
         b.wrap_items = WRAP_REPAIR_MAX;
-        b.wrap_mode = a.repair ? WRAP_REPAIR : (a.n_items <= WRAP_BUILD_MAX ? WRAP_OWN : WRAP_HANDED);
+        // (by the size of the whole build, of which `a` may be a piece: the pieces run side by side)
+        b.wrap_mode = a.repair ? WRAP_REPAIR : (c->n <= WRAP_BUILD_MAX ? WRAP_OWN : WRAP_HANDED);
         const bool short_lists = a.repair && a.n_items <= WRAP_REPAIR_MAX;   // (k_wrap takes them whole)
         if (b.wrap_mode != WRAP_OWN && !short_lists) {
             if ((e = launch_star(b, mode, c->sms, &c->launches, s)) != cudaSuccess) return e;

@@ -292,3 +292,23 @@ def test_narrow_boxes(width, cell, rebuild):
             a = _rings(p, boxes[part], cell, False, sizes=sizes[part], moved=moved, fp64=fp64)
             assert torch.equal(a[1], b[1])
             assert torch.equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("pieces", [1, 2, 8])
+def test_pieces_of_a_large_build(pieces):
+    # a build of 100,000 points in pieces (12,500 points each in 8): every piece in two launches of
+    # k_star and one of k_wrap, and the rings of the whole
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayGPU
+
+    n = 100_000
+    L = float(np.sqrt(n))
+    P = torch.from_numpy(W.uniform_points(n, L, 95)).cuda()
+    out, launches = [], []
+    for budget in (1024, 255):
+        d = DelaunayGPU(n, 24, 1.0, (L, L))
+        d.setDeferredOverlap(pieces)
+        d.setWorkBudget(budget)
+        out.append(d.globalDelaunayTriangulation(P))
+        launches.append(d.stats()["launches"])
+    assert launches[0] == launches[1] + 2 * pieces
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
