@@ -64,10 +64,21 @@ constexpr int SPILL_EDGES_PER_SM = 64;
 // Work lists of at most this many points per SM go to the warp-per-point kernel whole (two
 // points per resident warp)
 constexpr int WARP_ITEMS_PER_SM = 16;
-// Up to this many points a warp per point throughout (at 20,000 / 40,000 / 64,000: a build of 30,000
-// points 160 / 144 / 145 us, of 50,000 points 165 / 165 / 196 us; the 4M repair, whose rounds hold
-// 27,000 and 32,000 points, 1548 / 1506 / 1500 us, the 1M one with 45,000 and 59,000 882 / 885 / 981)
-constexpr int WRAP_BUILD_MAX = 40000;
+// Builds of up to WRAP_BUILD_MAX points go to the warp-per-point hull kernel whole; those of up to
+// STAR_ONCE_MAX take the first stage's first pass, and that kernel after it for every point that
+// is left (a fourth of a uniform set): a second pass is a launch as long as its longest chain.
+// Microseconds a build, warp per point / first pass alone / both passes:
+//   uniform points      10,000 110 / 112 / 158, 14,000 117 / 111 / 156, 39,600 173 / 130 / 161,
+//                       60,000 -- / 145 / 171, 130,000 -- / 210 / 203
+//   jittered squares    10,000 104 / 99 / 102, 14,000 110 / 86 / 90, 39,600 165 / 95 / 99,
+//                       130,000 -- / 126 / 124
+//   rhombic cells       10,000 110 / 124 / 161, 14,000 123 / 125 / 159, 39,600 185 / 163 / 174,
+//                       60,000 -- / 193 / 184
+constexpr int WRAP_BUILD_MAX = 12000;
+constexpr int STAR_ONCE_MAX = 48000;
+// Repair lists of up to this many points go to that kernel whole (at 20,000 / 40,000 / 64,000: the
+// 4M repair, whose rounds hold 27,000 and 32,000 points, 1548 / 1506 / 1500 us, the 1M one with
+// 45,000 and 59,000 882 / 885 / 981)
 constexpr int WRAP_REPAIR_MAX = 40000;
 constexpr int MAX_DEFER_CHUNKS = 8;   // slot chunks of an overlapped global build (dgt_set_deferred_overlap)
 constexpr int MAX_FLIP_ROUNDS = 24; // flip rounds of a checked call before the rest is rebuilt
@@ -461,7 +472,7 @@ RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int str
     a.second_rings[0] = c->flip0.as<int>();
     a.second_rings[1] = c->flip1.as<int>();
     a.second_split = c->n / 4;   // 64-byte rings in 16 bytes a point
-    a.second_cap = 2 * a.second_split;
+    a.second_cap = c->n <= STAR_ONCE_MAX ? 0 : 2 * a.second_split;
     a.second_base = 0;
     a.star_small = c->star_small;
     a.skin = &c->st.as<DevStatus>()->skin;
@@ -473,8 +484,9 @@ RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int str
 }
 
 // The rings of `a`'s points.  Large sets of points: the first stage with a thread per point
-// (k_star), then with a warp per point (k_wrap) what that could not finish; up to WRAP_BUILD_MAX
-// (repair: WRAP_REPAIR_MAX) points: k_wrap alone, whose latency is far shorter.  What is left goes
+// (k_star; up to STAR_ONCE_MAX points one pass of it), then with a warp per point (k_wrap) what that
+// could not finish; up to WRAP_BUILD_MAX (repair: WRAP_REPAIR_MAX) points: k_wrap alone, whose
+// latency is far shorter.  What is left goes
 // to the incremental warp kernel (exactly cocircular candidates, circles past half the box, sets
 // of a few cells).  Work budgets too small for the first stage's scans and the kernel shapes with
 // a group of lanes per point leave every point to the incremental kernels instead; the kernel

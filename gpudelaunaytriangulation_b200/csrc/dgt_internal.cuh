@@ -237,12 +237,12 @@ struct RingArgs {
     // points the first stage (dgt_star.cu) hands to the warp-per-point hull kernel (dgt_wrap.cu)
     int *star_list;
     int *star_count;
-    // global builds: slots its first pass could not certify, at most second_cap, and their rings,
-    // 16 words each: entry k is number second_base + k over the two arrays, the first of which holds
-    // second_split.  No room (0): both passes run in one launch
     int star_small;    // 1: every set's windows span few enough slots for 16-bit offsets (dgt_star.cu)
     int wrap_mode;     // which points k_wrap takes (WRAP_*)
     int wrap_items;    // repair: lists of at most this many points go to k_wrap whole
+    // global builds: slots its first pass could not certify, at most second_cap, and their rings,
+    // 16 words each: entry k is number second_base + k over the two arrays, the first of which holds
+    // second_split.  What finds no room goes to star_list; none at all (0): no second pass
     int *second_list;
     int *second_count;
     int *second_rings[2];

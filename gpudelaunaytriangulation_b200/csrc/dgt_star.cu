@@ -795,7 +795,7 @@ cudaError_t launch_star_g(const RingArgs &a, int sms, int *launches, cudaStream_
     cudaError_t e;
     if (sizeof(T) == 4 && a.star_small) e = launch_star_t<T, STAR_FIRST, false, GEN, sizeof(T) == 4>(a, sms, s);
     else e = launch_star_t<T, STAR_FIRST, false, GEN, false>(a, sms, s);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || a.second_cap <= 0) return e;
     *launches += 1;
     return launch_star_t<T, STAR_SECOND, false, GEN, false>(a, sms, s);
 }
