@@ -123,6 +123,7 @@ struct dgt_context {
     int graph_flip_rounds = ASYNC_FLIP_ROUNDS;   // flip rounds of unsynchronised calls
     bool binned = false;   // the cell lists hold a binning of the current grid
     int star_small = 0;    // see RingArgs
+    bool narrow = false;   // the incremental kernels throughout (plan_grid)
     int flip_cap = 0;
     // global builds in this many pieces of the cell order, each on a stream of its own with
     // the points it defers (1: the whole build, then the deferred points)
@@ -270,6 +271,38 @@ void plan_general_set(SetDesc &S, const double m[4], double a, int ns)
     S.star_win = star_window(S.per_cell);
 }
 
+// Whether so many points lie in narrow boxes that the incremental kernels are the faster ones for
+// all.  The hull kernels leave a point to the incremental warp kernel if a circle of it passes half
+// the box: for a uniform set w mean spacings wide a share of 1.4 (1 + x) exp(-x), x = pi w^2 / 16
+// (the tail of the circumradius; measured 0.19, 0.041, 0.0059, 0.00064, 0.00005 at w = 4.2 to 8.2),
+// and every point of a grid with less than 4 cells on an axis (unless its cells are so dense that a
+// thread's scan of them takes as long).  The first stage also leaves to the warp-per-point kernel
+// the sets too narrow for its windows.  A deferred point costs 0.08 us behind the 36 us of the
+// first, a point of the other kind 2.2 ns in a set of more than WRAP_BUILD_MAX; what the hull
+// kernels save is 65 us, over 60,000 points 1.1 ns a point.  Strips of uniform points, hull against
+// incremental kernels: w = 3.2 and 3,000 / 100,000 points 296 / 140 and 8,954 / 250 us, 4.2 144 / 130
+// and 2,487 / 249, 5.2 116 / 144 and 704 / 269, 6.2 107 / 140 and 281 / 284; 100,000 points in
+// squares of 16 sites 336 / 113.
+bool narrow_sets(const dgt_context *c)
+{
+    double deferred = 0.0, unstarred = 0.0;
+    for (int s = 0; s < c->num_sets; ++s) {
+        const SetDesc &S = c->sets[s];
+        double w = std::min(S.Lx, S.Ly), area = S.Lx * S.Ly;
+        if (c->general) {
+            const double *g = &c->gboxes[4 * (size_t)s];
+            area = std::fabs(g[0] * g[3] - g[1] * g[2]);
+            w = area / std::max(std::hypot(g[0], g[2]), std::hypot(g[1], g[3]));
+        }
+        const int few = std::min(S.xsize, S.ysize);
+        const double x = 3.14159265 / 16.0 * w * w * S.n / area;
+        if (few >= 4) deferred += S.n * std::min(1.0, 1.4 * (1.0 + x) * std::exp(-x));
+        else if (S.per_cell <= 16.0f) deferred += S.n;
+        if (few < S.star_win + 1) unstarred += S.n;
+    }
+    return 36.0 + 0.08 * deferred + (c->n > WRAP_BUILD_MAX ? 0.0022 * unstarred : 0.0) > std::max(65.0, 0.0011 * c->n);
+}
+
 // cell grid of every set from the requested cell edge
 int plan_grid(dgt_context *c)
 {
@@ -323,7 +356,7 @@ int plan_grid(dgt_context *c)
         S.n = ns;
         S.V = (float)pow2_at_least(std::max(Lx, Ly));
         S.per_cell = (float)(ns / ((double)xs * ys));
-    S.star_win = star_window(S.per_cell);
+        S.star_win = star_window(S.per_cell);
         blocks += set_block_grid(S, (int)blocks);
         cells += (long long)xs * ys;
         pbase += ns;
@@ -333,6 +366,7 @@ int plan_grid(dgt_context *c)
     c->star_small = 1;
     for (const SetDesc &S : c->sets)
         if ((double)S.per_cell * S.xsize * (S.star_win / 2 + 1) > 16000.0) c->star_small = 0;
+    c->narrow = narrow_sets(c);
     c->total_cells = (int)cells;
     c->total_blocks = (int)blocks;
     return DGT_OK;
@@ -488,8 +522,8 @@ RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int str
 // could not finish; up to WRAP_BUILD_MAX (repair: WRAP_REPAIR_MAX) points: k_wrap alone, whose
 // latency is far shorter.  What is left goes
 // to the incremental warp kernel (exactly cocircular candidates, circles past half the box, sets
-// of a few cells).  Work budgets too small for the first stage's scans and the kernel shapes with
-// a group of lanes per point leave every point to the incremental kernels instead; the kernel
+// of a few cells).  Work budgets too small for the first stage's scans, the kernel shapes with a
+// group of lanes per point and narrow boxes leave every point to the incremental kernels instead; the kernel
 // shape applies to those of global triangulations, the rebuild rounds take the default shape.
 cudaError_t run_rings(dgt_context *c, const RingArgs &a, cudaStream_t s, PhaseTimer *build_timer = nullptr)
 {
@@ -499,7 +533,7 @@ cudaError_t run_rings(dgt_context *c, const RingArgs &a, cudaStream_t s, PhaseTi
     cudaError_t e = cudaSuccess;
     RingArgs b = a;
     c->launches += any + 1;
-    if (c->work_budget >= STAR_MIN_BUDGET && kernel_shape_lanes(shape) == 1) {
+    if (c->work_budget >= STAR_MIN_BUDGET && kernel_shape_lanes(shape) == 1 && !c->narrow) {
         b.wrap_items = WRAP_REPAIR_MAX;
         // (by the size of the whole build, of which `a` may be a piece: the pieces run side by side)
         b.wrap_mode = a.repair ? WRAP_REPAIR : (c->n <= WRAP_BUILD_MAX ? WRAP_OWN : WRAP_HANDED);

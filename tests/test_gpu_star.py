@@ -268,30 +268,55 @@ def test_big_rebuild_rounds(fp64, sigma):
     _same_big(pts, tuple(m.reshape(-1)), 1.0, moved=pts + sigma * W.normal_pairs(198, n), fp64=fp64)
 
 
-@pytest.mark.parametrize("width", [4.7, 5.2, 6.2])
-@pytest.mark.parametrize("cell", [0.3, 0.6, 1.0])
+def _strips(width, sizes, seed):
+    boxes = np.stack([np.full(len(sizes), width), sizes / width], axis=1)
+    return np.concatenate([W.uniform_points(int(k), width, seed + i, float(b[1]))
+                           for i, (k, b) in enumerate(zip(sizes, boxes))]), boxes
+
+
 @pytest.mark.parametrize("rebuild", [False, True])
-def test_narrow_boxes(width, cell, rebuild):
-    # circles close to half the box and past it: windows over the whole short axis (where circles
-    # pass half the box, flag 32, the nearest images still give one answer)
-    sizes = np.arange(60, 360)
-    boxes = np.stack([np.full(300, width), sizes / width], axis=1)
-    pts = np.concatenate([W.uniform_points(int(k), width, 800 + i, float(b[1]))
-                          for i, (k, b) in enumerate(zip(sizes, boxes))])
-    assert len(pts) > 48_000
-    low = sizes.cumsum()[150]
-    for part in (slice(0, 150), slice(0, 300)):   # in one pass of k_star and in two
-        p = pts[:low - sizes[150]] if part.stop == 150 else pts
-        moved = None
-        if rebuild:
-            L = np.repeat(boxes[part], sizes[part], axis=0)
-            moved = np.mod(p + 0.2 * W.normal_pairs(801, len(p)), L)
-            moved = np.where(moved >= L, 0.0, moved)
-        b = _rings(p, boxes[part], cell, True, sizes=sizes[part], moved=moved)
-        for fp64 in (False, True):
-            a = _rings(p, boxes[part], cell, False, sizes=sizes[part], moved=moved, fp64=fp64)
-            assert torch.equal(a[1], b[1])
-            assert torch.equal(a[0], b[0])
+@pytest.mark.parametrize("width", [4.7, 5.2, 6.2])
+@pytest.mark.parametrize("cell", [0.3, 0.45, 0.6, 0.8, 1.0])
+@pytest.mark.parametrize("big", [8_000, 60_000])
+def test_narrow_boxes(big, cell, width, rebuild):
+    # circles close to half the box and past it (where circles pass half the box, flag 32, the
+    # nearest images still give one answer): windows over the whole short axis.  Beside a large set,
+    # so that the hull kernels are taken, of up to 12,000 points and more
+    sizes = np.arange(60, 150, 3)
+    pts, boxes = _strips(width, sizes, 800)
+    L = float(np.sqrt(big))
+    pts = np.concatenate([pts, W.uniform_points(big, L, 802)])
+    sizes = np.append(sizes, big)
+    boxes = np.concatenate([boxes, [[L, L]]])
+    moved = None
+    if rebuild:
+        every = np.repeat(boxes, sizes, axis=0)
+        moved = np.mod(pts + 0.2 * W.normal_pairs(801, len(pts)), every)
+        moved = np.where(moved >= every, 0.0, moved)
+    b = _rings(pts, boxes, cell, True, sizes=sizes, moved=moved)
+    for fp64 in (False, True):
+        a = _rings(pts, boxes, cell, False, sizes=sizes, moved=moved, fp64=fp64)
+        assert torch.equal(a[1], b[1])
+        assert torch.equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("width,sizes", [(2.5, [12_000]), (4.2, [3_000]), (4.2, [60_000]), (5.2, [100_000]),
+                                         (4.0, [16] * 2500), (5.0, [25] * 1600)])
+def test_mostly_narrow_boxes(width, sizes):
+    # sets whose circles pass half the box by the thousand: a thread per point, not a warp each
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayBatch
+
+    sizes = np.array(sizes)
+    if len(sizes) == 1:
+        pts, boxes = _strips(width, sizes, 810)
+    else:
+        pts = np.concatenate([W.square_lattice(int(k), 0.25, 810 + i)[0] for i, k in enumerate(sizes)])
+        boxes = np.full((len(sizes), 2), width)
+    d = DelaunayBatch(sizes, boxes, 24, 1.0)
+    d.globalDelaunayTriangulation(torch.from_numpy(pts).cuda())
+    assert d.stats()["exact_points"] < len(pts) // 100
+    a, b = (_rings(pts, boxes, 1.0, inc, sizes=sizes) for inc in (False, True))
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
 
 
 @pytest.mark.parametrize("pieces", [1, 2, 8])
