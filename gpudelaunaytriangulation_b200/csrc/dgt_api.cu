@@ -76,10 +76,13 @@ constexpr int WARP_ITEMS_PER_SM = 16;
 //                       60,000 -- / 193 / 184
 constexpr int WRAP_BUILD_MAX = 12000;
 constexpr int STAR_ONCE_MAX = 48000;
-// Repair lists of up to this many points go to that kernel whole (at 20,000 / 40,000 / 64,000: the
-// 4M repair, whose rounds hold 27,000 and 32,000 points, 1548 / 1506 / 1500 us, the 1M one with
-// 45,000 and 59,000 882 / 885 / 981)
-constexpr int WRAP_REPAIR_MAX = 40000;
+// The same for the lists of a repair's rounds, whose length the kernels read on the device (one pass
+// up to STAR_ONCE_MAX points; rebuild-only repairs of 100,000 / 250,000 jittered squares whose
+// lists hold some 35,000 points: 238 / 215 us with a warp per point up to 40,000, 166 / 190 us so).
+// Sets of up to WRAP_SHORT_MAX points leave the first stage out: a launch of it that finds a short
+// list costs 3 us a round.
+constexpr int WRAP_REPAIR_MAX = 20000;
+constexpr int WRAP_SHORT_MAX = 40000;
 constexpr int MAX_DEFER_CHUNKS = 8;   // slot chunks of an overlapped global build (dgt_set_deferred_overlap)
 constexpr int MAX_FLIP_ROUNDS = 24; // flip rounds of a checked call before the rest is rebuilt
 constexpr int ASYNC_FLIP_ROUNDS = 3; // default flip rounds of an unsynchronised call (best of 1-10 for MD steps at sigma 0.01)
@@ -519,8 +522,8 @@ RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int str
 
 // The rings of `a`'s points.  Large sets of points: the first stage with a thread per point
 // (k_star; up to STAR_ONCE_MAX points one pass of it), then with a warp per point (k_wrap) what that
-// could not finish; up to WRAP_BUILD_MAX (repair: WRAP_REPAIR_MAX) points: k_wrap alone, whose
-// latency is far shorter.  What is left goes
+// could not finish; up to WRAP_BUILD_MAX points (repair: lists of WRAP_REPAIR_MAX): k_wrap alone,
+// whose latency is far shorter.  What is left goes
 // to the incremental warp kernel (exactly cocircular candidates, circles past half the box, sets
 // of a few cells).  Work budgets too small for the first stage's scans, the kernel shapes with a
 // group of lanes per point and narrow boxes leave every point to the incremental kernels instead; the kernel
@@ -534,10 +537,11 @@ cudaError_t run_rings(dgt_context *c, const RingArgs &a, cudaStream_t s, PhaseTi
     RingArgs b = a;
     c->launches += any + 1;
     if (c->work_budget >= STAR_MIN_BUDGET && kernel_shape_lanes(shape) == 1 && !c->narrow) {
-        b.wrap_items = WRAP_REPAIR_MAX;
+        const bool short_lists = a.repair && a.n_items <= WRAP_SHORT_MAX;   // (k_wrap takes them whole)
+        b.wrap_items = short_lists ? a.n_items : WRAP_REPAIR_MAX;
+        b.star_once = STAR_ONCE_MAX;
         // (by the size of the whole build, of which `a` may be a piece: the pieces run side by side)
         b.wrap_mode = a.repair ? WRAP_REPAIR : (c->n <= WRAP_BUILD_MAX ? WRAP_OWN : WRAP_HANDED);
-        const bool short_lists = a.repair && a.n_items <= WRAP_REPAIR_MAX;   // (k_wrap takes them whole)
         if (b.wrap_mode != WRAP_OWN && !short_lists) {
             if ((e = launch_star(b, mode, c->sms, &c->launches, s)) != cudaSuccess) return e;
             b.count_round = 0;

@@ -240,6 +240,7 @@ struct RingArgs {
     int star_small;    // 1: every set's windows span few enough slots for 16-bit offsets (dgt_star.cu)
     int wrap_mode;     // which points k_wrap takes (WRAP_*)
     int wrap_items;    // repair: lists of at most this many points go to k_wrap whole
+    int star_once;     // repair: lists of at most this many points take k_star's first pass only
     // global builds: slots its first pass could not certify, at most second_cap, and their rings,
     // 16 words each: entry k is number second_base + k over the two arrays, the first of which holds
     // second_split.  What finds no room goes to star_list; none at all (0): no second pass

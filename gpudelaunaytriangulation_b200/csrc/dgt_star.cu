@@ -716,6 +716,7 @@ __global__ void __launch_bounds__(SMALL ? 128 : STAR_BLOCK) k_star(RingArgs A)
         atomicMax(&A.st->rounds, A.round + 1);
     }
     if (IDX && n <= A.wrap_items) return;   // a short list: k_wrap takes it
+    const int mode = IDX && n <= A.star_once ? STAR_FIRST : MODE;
     if ((int)blockIdx.x * B >= n) return;
     for (int base = blockIdx.x * B; base < n; base += gridDim.x * B) {
         const int it = base + t;
@@ -730,7 +731,7 @@ __global__ void __launch_bounds__(SMALL ? 128 : STAR_BLOCK) k_star(RingArgs A)
         Star<T, IDX, GEN, SMALL, CHECK> b(A, S, M, p, IDX ? pid : slot);
         if (act && !IDX) pid = __ldg(&A.sidx[slot]);
         if (MODE == STAR_SECOND && act) b.load_ring(second_ring(A, it));
-        b.run(MODE, act);
+        b.run(mode, act);
         if (act) {
             StarRing<T, SMALL> ring{ M, t };
             if (b.status == S_OK) {

@@ -161,7 +161,7 @@ def _build_big(pts, box, cell, incremental, fp64=False, sizes=None, moved=None, 
         d.testAndRepairDelaunayTriangulation(P, tri, nn)
         again = d.stats()
         assert again["mismatches"] == 0 and again["error_flags"] & ~32 == 0, again
-        assert again["flagged"] > 40_000   # the first round's list is k_star's
+        assert again["flagged"] > 20_000   # the first round's list is k_star's
         tri.view(len(pts), -1).masked_fill_(torch.arange(stride, device="cuda") >= nn[:, None], 0)
     return tri, nn, st
 
@@ -257,9 +257,9 @@ def test_big_batch():
 
 @pytest.mark.parametrize("fp64", [False, True])
 @pytest.mark.parametrize("sigma", [0.1, 0.3])
-def test_big_rebuild_rounds(fp64, sigma):
-    # lists of more than 40,000 points, with kept (0.1) and new cell lists
-    n = 90_000
+@pytest.mark.parametrize("n", [46_000, 90_000])
+def test_big_rebuild_rounds(n, fp64, sigma):
+    # lists of more than 20,000 points (one pass) and 48,000 (both), with kept (0.1) and new cell lists
     L = float(np.sqrt(n))
     pts = W.uniform_points(n, L, 195)
     _same_big(pts, (L, L), 1.0, moved=W.displace(pts, sigma, L, L, 196), fp64=fp64)
