@@ -166,6 +166,103 @@ __device__ __noinline__ int settle_angles(StarMem<T, SMALL> *M, int t, int n, un
     return out;
 }
 
+// the slot (or index) of the candidate at place k of a column
+template <typename T, bool SMALL>
+__device__ __forceinline__ int star_slot(const StarMem<T, SMALL> &M, int t, const SetDesc &S, int self, int k)
+{
+    if (!SMALL) return M.s[k][t];
+    int v = self + M.s[k][t];
+    if (v < S.point_base) v += S.n;
+    else if (v >= S.point_base + S.n) v -= S.n;
+    return v;
+}
+
+// How far the circles of a ring reach: extents along the cell axes (twice those of the circles) and
+// the largest diameter; good: all of them are bounded and well conditioned
+template <typename T, bool GEN>
+struct Reach {
+    typedef typename Prec<T>::T2 V2;
+    T sx, sy, g11, g12, g21, g22;
+    T ulo = Prec<T>::inf(), uhi = -Prec<T>::inf(), vlo = Prec<T>::inf(), vhi = -Prec<T>::inf(), wmax = (T)0;
+    bool good = true;
+    __device__ __forceinline__ Reach(const SetDesc &S)
+        : sx(GEN ? (T)S.gnx : (T)S.icw), sy(GEN ? (T)S.gny : (T)S.ich), g11((T)S.g11), g12((T)S.g12), g21((T)S.g21),
+          g22((T)S.g22)
+    {
+    }
+    // the circle through p and neighbours with the inverted offsets b and c (eb, ec: their err1)
+    __device__ __forceinline__ void add(V2 b, V2 c, T eb, T ec)
+    {
+        const T g = b.x * c.y - b.y * c.x;
+        // relative error of g below 24u 2^9 (2^-10.4 in float), of the pole below 2^-9.4
+        // (eb and ec are the one-norms times 16u)
+        good &= g > ((T)0.001953125 / ((T)256 * Prec<T>::u() * Prec<T>::u())) * eb * ec;
+        const T ig = rcp_fast(g);
+        const T wx = (c.y - b.y) * ig, wy = (b.x - c.x) * ig;
+        const T w2 = wx * wx + wy * wy;
+        const T hw = sqrt_over(w2) * (T)1.00390625;   // 1 + 2^-8
+        wmax = hw > wmax ? hw : wmax;
+        const T uc = GEN ? g11 * wx + g12 * wy : wx * sx, vc = GEN ? g21 * wx + g22 * wy : wy * sy;
+        const T hu = hw * sx, hv = hw * sy;
+        ulo = fmin(ulo, uc - hu);
+        uhi = fmax(uhi, uc + hu);
+        vlo = fmin(vlo, vc - hv);
+        vhi = fmax(vhi, vc + hv);
+    }
+};
+
+// Ring vertices whose turns are unsure (bit k: the k-th), in float64.  A vertex at a right turn is
+// interior, as in the pass over the stack, and leaves the ring; its neighbours' turns are looked at
+// again.  The ring's new length and reach (good: false too if a turn is not decided).
+// Near-cocircular lattices need it, half of whose diagonals stay on the stack (handing such points on
+// instead: 62,500 squares with a jitter of 1e-6 354 us, 111 in the incremental kernels, 119 so); out of
+// line, since it is rare elsewhere.
+template <typename T, bool GEN> struct Settled {
+    Reach<T, GEN> R;
+    int m;
+    unsigned u32, u64, mism;
+};
+template <typename T, bool GEN, bool SMALL>
+__device__ __noinline__ Settled<T, GEN> settle_ring(StarMem<T, SMALL> *M, int t, const SetDesc *S, const double2 *P, double2 p,
+                                                    int self, int m, unsigned unsure)
+{
+    auto ord = [&](int k) { return M->o[k + 1][t]; };
+    Settled<T, GEN> r{ Reach<T, GEN>(*S), m, 0, 0, 0 };
+    while (unsure) {
+        const int k = 31 - __clz(unsure);
+        unsure ^= 1u << k;
+        const int ka = ord(k > 0 ? k - 1 : m - 1), kb = ord(k), kc = ord(k + 1 < m ? k + 1 : 0);
+        const typename Prec<T>::T2 a = M->q[ka][t], b = M->q[kb][t], c = M->q[kc][t];
+        T o, bnd;
+        turn<T>(a, b, c, err1<T>(a), err1<T>(b), err1<T>(c), o, bnd);
+        const int e = star_recheck<GEN, false>(P, S, p, star_slot(*M, t, *S, self, ka), star_slot(*M, t, *S, self, kb),
+                                               star_slot(*M, t, *S, self, kc));
+        if (o > bnd) {   // (check mode, and neighbours of one that left)
+            r.mism += e < 0;
+            continue;
+        }
+        ++r.u32;
+        r.u64 += e == 0;
+        if (e > 0) continue;
+        if (e < 0) {
+            for (int j = k; j + 1 < m; ++j) M->o[j + 1][t] = M->o[j + 2][t];
+            --m;
+        }
+        if (e == 0 || m < 3) {
+            r.R.good = false;
+            return r;
+        }
+        const unsigned below = (1u << k) - 1u;
+        unsure = (unsure & below) | ((unsure >> 1) & ~below) | 1u << (k > 0 ? k - 1 : m - 1) | 1u << (k < m ? k : 0);
+    }
+    r.m = m;
+    for (int k = 0; k < m; ++k) {
+        const typename Prec<T>::T2 b = M->q[ord(k)][t], c = M->q[ord(k + 1 < m ? k + 1 : 0)][t];
+        r.R.add(b, c, err1<T>(b), err1<T>(c));
+    }
+    return r;
+}
+
 template <typename T, bool IDX, bool GEN, bool SMALL, bool CHECK>
 struct Star {
     typedef Prec<T> PR;
@@ -197,14 +294,7 @@ struct Star {
     }
 
     // the candidate at place k
-    __device__ __forceinline__ int slot(int k) const
-    {
-        if (!SMALL) return M.s[k][t];
-        int v = self + M.s[k][t];
-        if (v < S.point_base) v += S.n;
-        else if (v >= S.point_base + S.n) v -= S.n;
-        return v;
-    }
+    __device__ __forceinline__ int slot(int k) const { return star_slot(M, t, S, self, k); }
     // candidate number k of the order / of the ring (the sentinel is number -1)
     __device__ __forceinline__ int ord(int k) { return M.o[k + 1][t]; }
     // W cells per axis: centred on the own cell (odd W), or on its half that holds p (even W)
@@ -486,13 +576,9 @@ struct Star {
     // verdict is wanted.
     __device__ __forceinline__ void certify(T r2, T dropped, bool leave, bool again, T &wmax)
     {
-        T ulo = PR::inf(), uhi = -PR::inf(), vlo = PR::inf(), vhi = -PR::inf();
-        wmax = (T)0;
-        const T g11 = (T)S.g11, g12 = (T)S.g12, g21 = (T)S.g21, g22 = (T)S.g22;
-        const T sx = GEN ? (T)S.gnx : (T)S.icw, sy = GEN ? (T)S.gny : (T)S.ich;
+        Reach<T, GEN> R(S);
         V2 a = M.q[ord(m - 1)][t], b = M.q[ord(0)][t];
         T ea = err1<T>(a), eb = err1<T>(b);
-        bool good = true;
         unsigned unsure = 0;
         for (int k = 0; k < m; ++k) {
             const V2 c = M.q[ord(k + 1 < m ? k + 1 : 0)][t];
@@ -500,21 +586,7 @@ struct Star {
             T o, bnd;
             turn<T>(a, b, c, ea, eb, ec, o, bnd);
             unsure |= (unsigned)!(o > bnd) << k;
-            const T g = b.x * c.y - b.y * c.x;
-            // relative error of g below 24u 2^9 (2^-10.4 in float), of the pole below 2^-9.4
-            // (eb and ec are the one-norms times 16u)
-            good &= g > ((T)0.001953125 / ((T)256 * PR::u() * PR::u())) * eb * ec;
-            const T ig = rcp_fast(g);
-            const T wx = (c.y - b.y) * ig, wy = (b.x - c.x) * ig;
-            const T w2 = wx * wx + wy * wy;
-            const T hw = sqrt_over(w2) * (T)1.00390625;   // 1 + 2^-8
-            wmax = hw > wmax ? hw : wmax;
-            const T uc = GEN ? g11 * wx + g12 * wy : wx * sx, vc = GEN ? g21 * wx + g22 * wy : wy * sy;
-            const T hu = hw * sx, hv = hw * sy;
-            ulo = fmin(ulo, uc - hu);
-            uhi = fmax(uhi, uc + hu);
-            vlo = fmin(vlo, vc - hv);
-            vhi = fmax(vhi, vc + hv);
+            R.add(b, c, eb, ec);
             a = b;
             b = c;
             ea = eb;
@@ -522,7 +594,17 @@ struct Star {
         }
         // turns of the ring the filter left open: in float64
         if (CHECK) unsure = m == 32 ? ~0u : (1u << m) - 1u;
-        if (good && unsure) good = settle_turns(unsure);
+        if (R.good && unsure) {
+            const Settled<T, GEN> r = settle_ring<T, GEN, SMALL>(&M, t, &S, IDX ? A.pos : A.spos, p, self, m, unsure);
+            R = r.R;
+            m = r.m;
+            u32 += r.u32;
+            u64 += r.u64;
+            mism += r.mism;
+        }
+        const T ulo = R.ulo, uhi = R.uhi, vlo = R.vlo, vhi = R.vhi;
+        const bool good = R.good;
+        wmax = R.wmax;
         if (!good || !(wmax < (T)1e15) || (dropped > (T)0 && !(wmax * wmax * dropped < (T)8))) {
             status = S_FAIL;
             return;
@@ -568,29 +650,6 @@ struct Star {
         }
         for (int k = 0; k < m; ++k)
             M.q[STAR_CAP - 1 - k][t] = PR::mk2((T)__int_as_float(M.s[SMALL ? 0 : 2 * k][t]), (T)__int_as_float(M.s[SMALL ? 0 : 2 * k + 1][t]));
-    }
-
-    // ring vertices whose turns are unsure: all left in float64?
-    __device__ __forceinline__ bool settle_turns(unsigned unsure)
-    {
-        bool good = true;
-        while (unsure && good) {
-            const int k = __ffs(unsure) - 1;
-            unsure &= unsure - 1u;
-            const int ka = ord(k > 0 ? k - 1 : m - 1), kb = ord(k), kc = ord(k + 1 < m ? k + 1 : 0);
-            const V2 a = M.q[ka][t], b = M.q[kb][t], c = M.q[kc][t];
-            T o, bnd;
-            turn<T>(a, b, c, err1<T>(a), err1<T>(b), err1<T>(c), o, bnd);
-            const int e = recheck(ka, kb, kc);
-            if (o > bnd) {   // (check mode)
-                mism += e < 0;
-            } else {
-                ++u32;
-                u64 += e == 0;
-                good = e > 0;
-            }
-        }
-        return good;
     }
 
     // the window of the first pass
@@ -702,7 +761,10 @@ struct Star {
 };
 
 template <typename T, int MODE, bool IDX, bool GEN, bool SMALL, bool CHECK>
-__global__ void __launch_bounds__(SMALL ? 128 : STAR_BLOCK) k_star(RingArgs A)
+// (SMALL in general boxes: without the bound 106 registers, four blocks per SM instead of five, and
+// 454 us for 1M points instead of 318; in rectangles it has 96 without one, and the bound makes 4M
+// points 2.06 -> 2.09 ms.  0: no bound, which is not the same as 1.)
+__global__ void __launch_bounds__(SMALL ? 128 : STAR_BLOCK, SMALL && GEN ? 5 : 0) k_star(RingArgs A)
 {
     __shared__ StarMem<T, SMALL> M;
     constexpr int B = StarMem<T, SMALL>::B;

@@ -337,3 +337,21 @@ def test_pieces_of_a_large_build(pieces):
         launches.append(d.stats()["launches"])
     assert launches[0] == launches[1] + 2 * pieces
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("n", [13_225, 62_500])
+@pytest.mark.parametrize("jitter", [1e-3, 1e-6, 1e-9])
+def test_near_cocircular_squares(jitter, n, fp64):
+    # the four corners of every square within rounding of a circle: the diagonals that are no edges
+    # are taken out of the ring by the float64 decision, in the first pass (25 candidates a point; a
+    # second kernel would scan as many again)
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayGPU
+
+    pts, L = W.square_lattice(n, phase=jitter, seed=5)
+    d = DelaunayGPU(n, 16, 1.0, (L, L))
+    d.setPrecision(not fp64)
+    d.globalDelaunayTriangulation(torch.from_numpy(pts).cuda())
+    st = d.stats()
+    assert st["candidates"] <= 26 * n and st["exact_points"] <= n // 1000, st
+    _same_big(pts, (L, L), 1.0, fp64=fp64)
