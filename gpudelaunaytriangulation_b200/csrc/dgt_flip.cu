@@ -312,17 +312,36 @@ __device__ __forceinline__ void flip_finish(const FlipArgs &A, DevCtl *ctl, int 
     }
 }
 
-// All rounds in one block, for sets whose candidates it can hold (FLIP_SMALL_MAX points): a round
-// is two barriers instead of two launches, each of which costs the latency of a whole chain of
-// gathers for a few hundred candidates (10,000 points, sigma 0.02: repair call 291 -> 234 us)
-template <bool GEN>
-__global__ void __launch_bounds__(512, 1) k_flip_small(FlipArgs A, DevCtl *ctl, int2 *list0, int2 *list1, int *count0,
-                                                       int *count1, int rounds, float max_skin)
+// a barrier of the cluster; what its threads wrote before it is seen by their reads after it
+__device__ __forceinline__ void cluster_barrier()
 {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// All rounds in one launch, for sets of at most FLIP_SMALL_MAX points: a round is two barriers
+// instead of two launches, each of which costs the latency of a whole chain of gathers for a few
+// hundred candidates.  Up to FLIP_BLOCK_MAX points one block, beyond a cluster of eight: a block
+// starts sooner and has the cheaper barriers, a cluster has eight times the gathers in flight for
+// the lists of larger sets and moves.  Microseconds a repair call in launches / one block / a
+// cluster: 1,000 points at sigma 0.03 339 / 162 / 187; 10,000 at 0.02, 0.06 and 0.15 393 / 251 / 257,
+// 481 / 443 / 327 and 513 / 536 / 387; 16,384 at 0.01, 0.06 and 0.15 301 / 198 / 190, 499 / 607 / 363
+// and 513 / 747 / 443.
+constexpr int FLIP_CLUSTER = 8;
+constexpr int FLIP_BLOCK_MAX = 10000;
+template <bool GEN, bool CLUSTER>
+__device__ __forceinline__ void flip_rounds(FlipArgs &A, DevCtl *ctl, int2 *list0, int2 *list1, int *count0, int *count1,
+                                            int rounds, float max_skin)
+{
+    auto barrier = []() {
+        if (CLUSTER) cluster_barrier();
+        else __syncthreads();
+    };
     const int ebase = *A.epoch_ptr + 1;
     const unsigned stamp0 = *A.stamp_ptr + 1;
+    const int block = blockIdx.x * blockDim.x, first = block + threadIdx.x, step = gridDim.x * blockDim.x;
     unsigned long long flips = 0;
     int r = 0;
+    // (every thread reads the same n: the same trips, the same barriers)
     for (;; ++r) {
         A.cur = r & 1 ? list1 : list0;
         A.next = r & 1 ? list0 : list1;
@@ -330,14 +349,28 @@ __global__ void __launch_bounds__(512, 1) k_flip_small(FlipArgs A, DevCtl *ctl, 
         A.next_count = r & 1 ? count0 : count1;
         const int n = min(__ldcg(A.cur_count), A.cap);
         if (n == 0 || r >= rounds) break;
-        if (threadIdx.x == 0) *A.next_count = 0;
-        flip_claim<GEN>(A, ebase, stamp0 + r, n, threadIdx.x, blockDim.x);
-        __syncthreads();
-        flip_apply<GEN>(A, ebase, stamp0 + r, n, 0, blockDim.x, flips);
-        __syncthreads();
+        if (first == 0) *A.next_count = 0;
+        flip_claim<GEN>(A, ebase, stamp0 + r, n, first, step);
+        barrier();
+        flip_apply<GEN>(A, ebase, stamp0 + r, n, block, step, flips);
+        barrier();
     }
     count_flips(A, flips);
-    flip_finish(A, ctl, ebase, min(__ldcg(A.cur_count), A.cap), threadIdx.x, blockDim.x, r, max_skin);
+    flip_finish(A, ctl, ebase, min(__ldcg(A.cur_count), A.cap), first, step, r, max_skin);
+}
+
+// (a kernel each: with cluster dimensions of one block a launch in a graph takes 3 us longer)
+template <bool GEN>
+__global__ void __launch_bounds__(512, 1) k_flip_small(FlipArgs A, DevCtl *ctl, int2 *list0, int2 *list1, int *count0,
+                                                       int *count1, int rounds, float max_skin)
+{
+    flip_rounds<GEN, false>(A, ctl, list0, list1, count0, count1, rounds, max_skin);
+}
+template <bool GEN>
+__global__ void __cluster_dims__(FLIP_CLUSTER, 1, 1) __launch_bounds__(512, 1)
+    k_flip_cluster(FlipArgs A, DevCtl *ctl, int2 *list0, int2 *list1, int *count0, int *count1, int rounds, float max_skin)
+{
+    flip_rounds<GEN, true>(A, ctl, list0, list1, count0, count1, rounds, max_skin);
 }
 
 __global__ void __launch_bounds__(256) k_flip_spill(FlipArgs A, DevCtl *ctl, int rounds, float max_skin)
@@ -370,8 +403,11 @@ cudaError_t launch_flip_spill(const FlipArgs &a, int rounds, DevCtl *ctl, float 
 cudaError_t launch_flip_small(const FlipArgs &a, int rounds, DevCtl *ctl, int2 *const lists[2], int *const counts[2],
                               float max_skin, cudaStream_t s)
 {
-    if (a.general) k_flip_small<true><<<1, 512, 0, s>>>(a, ctl, lists[0], lists[1], counts[0], counts[1], rounds, max_skin);
-    else k_flip_small<false><<<1, 512, 0, s>>>(a, ctl, lists[0], lists[1], counts[0], counts[1], rounds, max_skin);
+    auto launch = [&](auto *kernel, int blocks) {
+        kernel<<<blocks, 512, 0, s>>>(a, ctl, lists[0], lists[1], counts[0], counts[1], rounds, max_skin);
+    };
+    if (a.n <= FLIP_BLOCK_MAX) launch(a.general ? k_flip_small<true> : k_flip_small<false>, 1);
+    else launch(a.general ? k_flip_cluster<true> : k_flip_cluster<false>, FLIP_CLUSTER);
     return cudaGetLastError();
 }
 

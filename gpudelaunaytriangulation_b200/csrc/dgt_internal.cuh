@@ -390,7 +390,8 @@ cudaError_t launch_flip_round(const FlipArgs &a, int round, int sms, cudaStream_
 // leftover candidates to the rebuild list; advances the context's flip stamp by rounds + 1;
 // max_skin >= 0: decides whether the cell lists can stay (launch_refresh's decision)
 cudaError_t launch_flip_spill(const FlipArgs &a, int rounds, DevCtl *ctl, float max_skin, int sms, cudaStream_t s);
-// sets of at most FLIP_SMALL_MAX points: up to `rounds` rounds and the spill in one launch
+// sets of at most FLIP_SMALL_MAX points: up to `rounds` rounds and the spill in one launch (of a block or
+// a cluster)
 constexpr int FLIP_SMALL_MAX = 16384;
 cudaError_t launch_flip_small(const FlipArgs &a, int rounds, DevCtl *ctl, int2 *const lists[2], int *const counts[2],
                               float max_skin, cudaStream_t s);

@@ -355,3 +355,37 @@ def test_near_cocircular_squares(jitter, n, fp64):
     st = d.stats()
     assert st["candidates"] <= 26 * n and st["exact_points"] <= n // 1000, st
     _same_big(pts, (L, L), 1.0, fp64=fp64)
+
+
+@pytest.mark.parametrize("n", [1000, 10_000, 10_001, 16_384])
+@pytest.mark.parametrize("sigma", [0.02, 0.15])
+@pytest.mark.parametrize("general", [False, True])
+def test_flip_rounds_of_small_sets(general, sigma, n):
+    # all flip rounds in one block or one cluster (long lists at the larger sigma), five moves in a
+    # row: the rings of a fresh build
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayGPU
+
+    L = float(np.sqrt(n))
+    m = np.array(HEX).reshape(2, 2) * float(np.sqrt(n / (np.sqrt(3.0) / 2.0)))
+    box = tuple(m.reshape(-1)) if general else (L, L)
+    pts = W.uniform_points(n, 1.0, 720 + n) @ m.T if general else W.uniform_points(n, L, 720 + n)
+    d = DelaunayGPU(n, 24, 1.0, box)
+    P = torch.from_numpy(np.ascontiguousarray(pts)).cuda()
+    tri, nn = d.globalDelaunayTriangulation(P)
+    flips = 0
+    for step in range(5):
+        pts = pts + sigma * W.normal_pairs(721 + step, n)
+        if not general:
+            pts = W.wrap(pts, L, L)
+        P.copy_(torch.from_numpy(pts))
+        d.testAndRepairDelaunayTriangulation(P, tri, nn)
+        flips += d.stats()["flips"]
+        assert d.stats()["error_flags"] == 0
+        fresh, k = DelaunayGPU(n, 24, 1.0, box).globalDelaunayTriangulation(P)
+        assert torch.equal(nn, k)
+        rows = torch.arange(24, device="cuda")[None, :] < k[:, None]
+        # (a repaired row may begin at another of its entries)
+        a, b = (torch.where(rows, t.view(n, -1), -1).sort(dim=1).values for t in (tri, fresh))
+        assert torch.equal(a, b)
+        assert d.validate(P, tri, nn)["valid"] == 1
+    assert flips > 0
