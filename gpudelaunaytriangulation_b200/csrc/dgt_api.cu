@@ -64,19 +64,8 @@ constexpr int SPILL_EDGES_PER_SM = 64;
 // Work lists of at most this many points per SM go to the warp-per-point kernel whole (two
 // points per resident warp)
 constexpr int WARP_ITEMS_PER_SM = 16;
-// Builds of up to WRAP_BUILD_MAX points go to the warp-per-point hull kernel whole; those of up to
-// STAR_ONCE_MAX take the first stage's first pass, and that kernel after it for every point that
-// is left (a fourth of a uniform set): a second pass is a launch as long as its longest chain.
-// Microseconds a build, warp per point / first pass alone / both passes:
-//   uniform points      10,000 110 / 112 / 158, 14,000 117 / 111 / 156, 39,600 173 / 130 / 161,
-//                       60,000 -- / 145 / 171, 130,000 -- / 210 / 203
-//   jittered squares    10,000 104 / 99 / 102, 14,000 110 / 86 / 90, 39,600 165 / 95 / 99,
-//                       130,000 -- / 126 / 124
-//   rhombic cells       10,000 110 / 124 / 161, 14,000 123 / 125 / 159, 39,600 185 / 163 / 174,
-//                       60,000 -- / 193 / 184
-constexpr int WRAP_BUILD_MAX = 12000;
-constexpr int STAR_ONCE_MAX = 48000;
-// The same for the lists of a repair's rounds, whose length the kernels read on the device (one pass
+// WRAP_BUILD_MAX's counterpart for the lists of a repair's rounds, whose length the kernels read on the
+// device (one pass
 // up to STAR_ONCE_MAX points; rebuild-only repairs of 100,000 / 250,000 jittered squares whose
 // lists hold some 35,000 points: 238 / 215 us with a warp per point up to 40,000, 166 / 190 us so).
 // Sets of up to WRAP_SHORT_MAX points leave the first stage out: a launch of it that finds a short
@@ -274,21 +263,10 @@ void plan_general_set(SetDesc &S, const double m[4], double a, int ns)
     S.star_win = star_window(S.per_cell);
 }
 
-// Whether so many points lie in narrow boxes that the incremental kernels are the faster ones for
-// all.  The hull kernels leave a point to the incremental warp kernel if a circle of it passes half
-// the box: for a uniform set w mean spacings wide a share of 1.4 (1 + x) exp(-x), x = pi w^2 / 16
-// (the tail of the circumradius; measured 0.19, 0.041, 0.0059, 0.00064, 0.00005 at w = 4.2 to 8.2),
-// and every point of a grid with less than 4 cells on an axis (unless its cells are so dense that a
-// thread's scan of them takes as long).  The first stage also leaves to the warp-per-point kernel
-// the sets too narrow for its windows.  A deferred point costs 0.08 us behind the 36 us of the
-// first, a point of the other kind 2.2 ns in a set of more than WRAP_BUILD_MAX; what the hull
-// kernels save is 65 us, over 60,000 points 1.1 ns a point.  Strips of uniform points, hull against
-// incremental kernels: w = 3.2 and 3,000 / 100,000 points 296 / 140 and 8,954 / 250 us, 4.2 144 / 130
-// and 2,487 / 249, 5.2 116 / 144 and 704 / 269, 6.2 107 / 140 and 281 / 284; 100,000 points in
-// squares of 16 sites 336 / 113.
+// the incremental kernels for all sets (HullLoad)?
 bool narrow_sets(const dgt_context *c)
 {
-    double deferred = 0.0, unstarred = 0.0;
+    HullLoad load;
     for (int s = 0; s < c->num_sets; ++s) {
         const SetDesc &S = c->sets[s];
         double w = std::min(S.Lx, S.Ly), area = S.Lx * S.Ly;
@@ -297,13 +275,9 @@ bool narrow_sets(const dgt_context *c)
             area = std::fabs(g[0] * g[3] - g[1] * g[2]);
             w = area / std::max(std::hypot(g[0], g[2]), std::hypot(g[1], g[3]));
         }
-        const int few = std::min(S.xsize, S.ysize);
-        const double x = 3.14159265 / 16.0 * w * w * S.n / area;
-        if (few >= 4) deferred += S.n * std::min(1.0, 1.4 * (1.0 + x) * std::exp(-x));
-        else if (S.per_cell <= 16.0f) deferred += S.n;
-        if (few < S.star_win + 1) unstarred += S.n;
+        load.add(S, w, area);
     }
-    return 36.0 + 0.08 * deferred + (c->n > WRAP_BUILD_MAX ? 0.0022 * unstarred : 0.0) > std::max(65.0, 0.0011 * c->n);
+    return load.narrow(c->n);
 }
 
 // cell grid of every set from the requested cell edge
@@ -365,10 +339,9 @@ int plan_grid(dgt_context *c)
         pbase += ns;
         if (cells > (1LL << 30)) return DGT_ERR_INVALID_ARGUMENT;
     }
-    // rows of a window in slots, half of the 16-bit range left for uneven densities
     c->star_small = 1;
     for (const SetDesc &S : c->sets)
-        if ((double)S.per_cell * S.xsize * (S.star_win / 2 + 1) > 16000.0) c->star_small = 0;
+        if (!star_fits_small(S)) c->star_small = 0;
     c->narrow = narrow_sets(c);
     c->total_cells = (int)cells;
     c->total_blocks = (int)blocks;

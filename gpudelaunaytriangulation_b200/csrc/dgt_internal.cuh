@@ -12,6 +12,8 @@
 // Point indices are global over the concatenated sets; the slots of set s are the range
 // [point_base, point_base + n) because cells are numbered set-major.
 #pragma once
+#include <algorithm>
+#include <cmath>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -374,6 +376,51 @@ inline int star_window(double per_cell)
     while (w > 3 && (double)w * w * per_cell > 26.0) --w;
     return w;
 }
+// rows of a window in slots fit 16-bit offsets, half of their range left for uneven densities
+inline bool star_fits_small(const SetDesc &S)
+{
+    return (double)S.per_cell * S.xsize * (S.star_win / 2 + 1) <= 16000.0;
+}
+// Builds of up to WRAP_BUILD_MAX points go to the warp-per-point hull kernel whole; those of up to
+// STAR_ONCE_MAX take the first stage's first pass, and that kernel after it for every point that
+// is left (a fourth of a uniform set): a second pass is a launch as long as its longest chain.
+// Microseconds a build, warp per point / first pass alone / both passes:
+//   uniform points      10,000 110 / 112 / 158, 14,000 117 / 111 / 156, 39,600 173 / 130 / 161,
+//                       60,000 -- / 145 / 171, 130,000 -- / 210 / 203
+//   jittered squares    10,000 104 / 99 / 102, 14,000 110 / 86 / 90, 39,600 165 / 95 / 99,
+//                       130,000 -- / 126 / 124
+//   rhombic cells       10,000 110 / 124 / 161, 14,000 123 / 125 / 159, 39,600 185 / 163 / 174,
+//                       60,000 -- / 193 / 184
+constexpr int WRAP_BUILD_MAX = 12000;
+constexpr int STAR_ONCE_MAX = 48000;
+// Whether so many points lie in narrow boxes that the incremental kernels are the faster ones for
+// all.  The hull kernels leave a point to the incremental warp kernel if a circle of it passes half
+// the box: for a uniform set w mean spacings wide a share of 1.4 (1 + x) exp(-x), x = pi w^2 / 16
+// (the tail of the circumradius; measured 0.19, 0.041, 0.0059, 0.00064, 0.00005 at w = 4.2 to 8.2),
+// and every point of a grid with less than 4 cells on an axis (unless its cells are so dense that a
+// thread's scan of them takes as long).  The first stage also leaves to the warp-per-point kernel
+// the sets too narrow for its windows.  A deferred point costs 0.08 us behind the 36 us of the
+// first, a point of the other kind 2.2 ns in a set of more than WRAP_BUILD_MAX; what the hull
+// kernels save is 65 us, over 60,000 points 1.1 ns a point.  Strips of uniform points, hull against
+// incremental kernels: w = 3.2 and 3,000 / 100,000 points 296 / 140 and 8,954 / 250 us, 4.2 144 / 130
+// and 2,487 / 249, 5.2 116 / 144 and 704 / 269, 6.2 107 / 140 and 281 / 284; 100,000 points in
+// squares of 16 sites 336 / 113.
+struct HullLoad {
+    double deferred = 0.0, unstarred = 0.0;
+    // width: the smallest distance between opposite sides of the set's box
+    void add(const SetDesc &S, double width, double area)
+    {
+        const int few = std::min(S.xsize, S.ysize);
+        const double x = 3.14159265 / 16.0 * width * width * S.n / area;
+        if (few >= 4) deferred += S.n * std::min(1.0, 1.4 * (1.0 + x) * std::exp(-x));
+        else if (S.per_cell <= 16.0f) deferred += S.n;
+        if (few < S.star_win + 1) unstarred += S.n;
+    }
+    bool narrow(int n) const
+    {
+        return 36.0 + 0.08 * deferred + (n > WRAP_BUILD_MAX ? 0.0022 * unstarred : 0.0) > std::max(65.0, 0.0011 * n);
+    }
+};
 // the one-ring kernel with `lanes` (4 or 8) lanes per point (dgt_group.cu)
 cudaError_t launch_build_group(const RingArgs &a, int mode, int sms, int lanes, cudaStream_t s);
 cudaError_t launch_deferred(const RingArgs &a, int sms, cudaStream_t s);

@@ -203,9 +203,24 @@ extern "C" int dgt_global_triangulation_noalloc(const double *d_points, int n, d
     r.defer_count = &d_st->defer_count;
     r.work_budget = DEFAULT_WORK_BUDGET;
     r.st = d_st;
-    // (a warp per point: at most 65,536 of them)
-    r.wrap_mode = WRAP_OWN;
-    if (launch_wrap(r, MODE_F32, sms, s) != cudaSuccess) return DGT_ERR_CUDA;
+    // The kernels that a context would choose (run_rings in dgt_api.cu), except that k_star always runs
+    // one pass: 65,536 uniform points 149 us, 205 us in the incremental kernels, 235 us with a warp per point
+    HullLoad load;
+    load.add(S, std::min(Lx, Ly), Lx * Ly);
+    if (load.narrow(n)) {
+        if (launch_build(r, MODE_F32, sms, 0, s) != cudaSuccess) return DGT_ERR_CUDA;
+    } else {
+        r.wrap_mode = n <= WRAP_BUILD_MAX ? WRAP_OWN : WRAP_HANDED;
+        if (r.wrap_mode == WRAP_HANDED) {
+            r.star_list = b.rank;   // (the binning is done with it)
+            r.star_count = &d_st->star_count;
+            r.second_count = &d_st->second_count;
+            r.star_small = star_fits_small(S) ? 1 : 0;
+            int launches = 0;
+            if (launch_star(r, MODE_F32, sms, &launches, s) != cudaSuccess) return DGT_ERR_CUDA;
+        }
+        if (launch_wrap(r, MODE_F32, sms, s) != cudaSuccess) return DGT_ERR_CUDA;
+    }
     if (launch_deferred(r, sms, s) != cudaSuccess) return DGT_ERR_CUDA;
 
     // status into host stack memory (pageable: no pinned buffer is allocated)

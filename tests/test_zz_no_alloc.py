@@ -163,3 +163,18 @@ def test_noalloc_reports_required_stride():
     assert code == N.DGT_OK
     rt, rk = with_context(pts, L, stride=need)
     assert same_rings(t, k, rt, rk)
+
+
+@pytest.mark.parametrize("n,width", [(12_000, None), (12_001, None), (3000, 3.2), (60_000, 4.2), (13_000, 8.2)])
+def test_noalloc_every_choice_of_kernels(n, width):
+    # a warp per point, the first stage and a warp per point, the incremental kernels (narrow boxes)
+    from gpudelaunaytriangulation_b200.delaunay import DelaunayGPU
+
+    Lx, Ly = (n / width, width) if width else (float(np.sqrt(n)),) * 2
+    pts = W.uniform_points(n, Lx, 19, Ly)
+    code, t, k, need = noalloc(pts, Lx, 64, Ly=Ly)
+    assert code == N.DGT_OK, N.lib().dgt_error_string(code)
+    d = DelaunayGPU(n, 64, 1.0, (Lx, Ly))
+    d.setWorkBudget(255)   # the incremental kernels
+    tri, nn = d.globalDelaunayTriangulation(torch.from_numpy(pts).cuda())
+    assert same_rings(t, k, tri.view(n, -1).cpu().numpy(), nn.cpu().numpy())
