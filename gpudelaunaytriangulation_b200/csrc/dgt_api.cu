@@ -493,6 +493,12 @@ RingArgs ring_args(dgt_context *c, const double *pts, int *tri, int *nn, int str
     return a;
 }
 
+// whether the hull kernels come first (run_rings), at a kernel shape
+bool hull_kernels(const dgt_context *c, int shape)
+{
+    return c->work_budget >= STAR_MIN_BUDGET && kernel_shape_lanes(shape) == 1 && !c->narrow;
+}
+
 // The rings of `a`'s points.  Large sets of points: the first stage with a thread per point
 // (k_star; up to STAR_ONCE_MAX points one pass of it), then with a warp per point (k_wrap) what that
 // could not finish; up to WRAP_BUILD_MAX points (repair: lists of WRAP_REPAIR_MAX): k_wrap alone,
@@ -509,7 +515,7 @@ cudaError_t run_rings(dgt_context *c, const RingArgs &a, cudaStream_t s, PhaseTi
     cudaError_t e = cudaSuccess;
     RingArgs b = a;
     c->launches += any + 1;
-    if (c->work_budget >= STAR_MIN_BUDGET && kernel_shape_lanes(shape) == 1 && !c->narrow) {
+    if (hull_kernels(c, shape)) {
         const bool short_lists = a.repair && a.n_items <= WRAP_SHORT_MAX;   // (k_wrap takes them whole)
         b.wrap_items = short_lists ? a.n_items : WRAP_REPAIR_MAX;
         b.star_once = STAR_ONCE_MAX;
@@ -1492,7 +1498,13 @@ int dgt_autotune(dgt_context *c, const double *d_points, int *d_tri, int *d_nn, 
             best_rel = rel;
         }
     }
+    if (rr == DGT_OK) {
+        set_relative_cell(c, best_rel);
+        rr = init_context(c);
+    }
     for (int shape = 1; shape < KERNEL_SHAPES && rr == DGT_OK; ++shape) {
+        // (where the hull kernels come first the shapes with a lane per point are one and the same)
+        if (hull_kernels(c, shape)) continue;
         float ms = 0;
         rr = trial(best_rel, shape, &ms);
         if (rr != DGT_OK) break;

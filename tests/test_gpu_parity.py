@@ -541,3 +541,19 @@ def test_exact_points_are_the_deferred_ones(n):
     d.globalDelaunayTriangulation(torch.from_numpy(pts).cuda())
     st = d.stats()
     assert st["points"] + st["exact_points"] == 2500 and st["exact_points"] > 0, st
+
+
+@pytest.mark.parametrize("n,budget,trials", [(20_000, 1024, 7), (9_000, 255, 11)])
+def test_autotune_tries_only_shapes_that_differ(n, budget, trials):
+    # five cell sizes and, where the hull kernels come first, the two shapes that replace them (the
+    # others name the same kernels); with a work budget that leaves them out all six others
+    L = float(np.sqrt(n))
+    P = torch.from_numpy(W.uniform_points(n, L, 114)).cuda()
+    tri = torch.zeros(20 * n, dtype=torch.int32, device="cuda")
+    nn = torch.zeros(n, dtype=torch.int32, device="cuda")
+    d = _dg()(n, 20, 1.0, (L, L))
+    d.setWorkBudget(budget)
+    res = d.autotune(P, tri, nn)
+    assert res["from_cache"] == 0 and res["trials"] == trials, res
+    assert res["shape"] in (0, 5, 6) or budget < 256, res
+    assert d.validate(P, tri, nn)["valid"] == 1
