@@ -359,9 +359,9 @@ int kernel_shape_block(int shape);
 int kernel_shape_lanes(int shape);
 cudaError_t launch_build(const RingArgs &a, int mode, int sms, int shape, cudaStream_t s);
 // The first stage of builds and rebuilds with a thread per point (dgt_star.cu); what it cannot
-// finish goes to a.star_list.  It scans at most some 200 cells and candidates a point, so a work
-// budget below STAR_MIN_BUDGET leaves every point to the incremental kernels.  (launches:
-// incremented by the kernels launched)
+// finish goes to a.star_list.  It scans some 200 cells and candidates a point at most where the
+// density is even, so a work budget below STAR_MIN_BUDGET leaves every point to the incremental
+// kernels.  (launches: incremented by the kernels launched)
 constexpr int STAR_MIN_BUDGET = 256;
 cudaError_t launch_star(const RingArgs &a, int mode, int sms, int *launches, cudaStream_t s);
 // The same with a warp per point (dgt_wrap.cu, a.wrap_mode); what it cannot finish goes to the

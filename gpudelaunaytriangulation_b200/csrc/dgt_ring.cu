@@ -55,7 +55,6 @@ __global__ void __launch_bounds__(BLOCK) k_build(RingArgs A)
         if (act) {
             if (A.worklist) {
                 pid = A.worklist[t];
-                if (pid < 0) pid = ~pid;   // too large a scan for the first stage
                 slot = A.slot_of[pid];
             } else {
                 slot = A.item_base + t;

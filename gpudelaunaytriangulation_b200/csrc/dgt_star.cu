@@ -1,5 +1,6 @@
-// One-ring construction from a bounded set of candidates (k_star): the first stage of every
-// build and rebuild; points it cannot finish go to the incremental kernels (dgt_ring.cu).
+// One-ring construction from a bounded set of candidates (k_star): the first stage of builds and
+// rebuilds of many points; what it cannot finish goes to the warp-per-point hull kernel
+// (dgt_wrap.cu), and only that kernel's leftovers to the incremental warp kernel (dgt_ring.cu).
 //
 // Inversion d -> d' = d / |d|^2 about the point p (all offsets relative to p) turns the circle
 // through p, a and b into the line through a' and b', and "d strictly inside that circle" into

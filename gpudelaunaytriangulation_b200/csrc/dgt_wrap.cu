@@ -8,7 +8,7 @@
 // left of the edge, so each accepted edge is a hull edge whatever the rounding of the slopes
 // (undecided turns go to float64 and exact arithmetic; an exactly cocircular candidate hands the
 // point on).  Afterwards one lane per edge computes its circle.  While some circle reaches out
-// of the window the window grows towards the circles' cells, at most doubling per pass, and only
+// of the window the window grows towards the circles' cells, at most tripling per pass, and only
 // candidates that may lie inside a circle join the ring for the next walk: a candidate outside
 // every circle stays outside, since the union of the circles only shrinks.  A ring that is open
 // in its first window takes four virtual corners along, like the incremental kernels.
@@ -272,15 +272,13 @@ struct Wrap {
             V2 v[K];
 #pragma unroll
             for (int j = 0; j < K; ++j) {
-                {
-                    v[j] = PR::mk2(c[j].x - a.x, c[j].y - a.y);
-                    const float u = (float)(a.x * v[j].y - a.y * v[j].x);
-                    const float slope = -(float)(a.x * v[j].x + a.y * v[j].y) * rcp_fast(u);
-                    const int k = lane + 32 * j;
-                    if (u > 0.0f && slope < best && k != ka && k < n) {
-                        best = slope;
-                        kb = k;
-                    }
+                v[j] = PR::mk2(c[j].x - a.x, c[j].y - a.y);
+                const float u = (float)(a.x * v[j].y - a.y * v[j].x);
+                const float slope = -(float)(a.x * v[j].x + a.y * v[j].y) * rcp_fast(u);
+                const int k = lane + 32 * j;
+                if (u > 0.0f && slope < best && k != ka && k < n) {
+                    best = slope;
+                    kb = k;
                 }
             }
             const unsigned key = kb >= 0 ? ordered(best) : FULL, least = __reduce_min_sync(FULL, key);
@@ -295,13 +293,11 @@ struct Wrap {
                 unsigned open = 0;
 #pragma unroll
                 for (int j = 0; j < K; ++j) {
-                    {
-                        // (turn() with the differences at hand)
-                        const int k = lane + 32 * j;
-                        const T o = ux * v[j].y - uy * v[j].x;
-                        const T bnd = (fabs(v[j].x) + fabs(v[j].y)) * eab + (lu * (ea + ec[j]) + PR::tiny());
-                        open |= (unsigned)(k < n && k != ka && k != kb && (!(o > bnd) || check)) << j;
-                    }
+                    // (turn() with the differences at hand)
+                    const int k = lane + 32 * j;
+                    const T o = ux * v[j].y - uy * v[j].x;
+                    const T bnd = (fabs(v[j].x) + fabs(v[j].y)) * eab + (lu * (ea + ec[j]) + PR::tiny());
+                    open |= (unsigned)(k < n && k != ka && k != kb && (!(o > bnd) || check)) << j;
                 }
                 ++tests;
                 unsigned lanes = __ballot_sync(FULL, open != 0);
@@ -346,8 +342,6 @@ struct Wrap {
         return -1;
     }
 
-    // (A window of three cells may scan WRAP_WORK candidates: dense cells, as of a clustered set at the
-    // mean spacing, 5,850 a point: 1M points 62 ms in the incremental kernels, 37 ms here.)
     // the whole construction; W_OK: lane k < m holds the ring's k-th entry in `out`
     __device__ __forceinline__ int run(int &out)
     {
@@ -375,6 +369,8 @@ struct Wrap {
             // what is there already: nothing, or the ring
             n = first ? 0 : m;
             const unsigned seen = cand;
+            // (a window of three cells may scan WRAP_WORK candidates: dense cells, as of a clustered set at
+            // the mean spacing, 5,850 a point: 1M points 62 ms in the incremental kernels, 37 ms here)
             const bool fits = gather(x0, x1, y0, y1, r2, filter, first && W > 3 ? 8 * WRAP_CAP : (int)WRAP_WORK);
             if (n > WRAP_CAP) return W_FAIL;
             if (cand > WRAP_WORK) return W_HEAVY;
