@@ -225,7 +225,7 @@ template <typename T, bool GEN> struct Settled {
 };
 template <typename T, bool GEN, bool SMALL>
 __device__ __noinline__ Settled<T, GEN> settle_ring(StarMem<T, SMALL> *M, int t, const SetDesc *S, const double2 *P, double2 p,
-                                                    int self, int m, unsigned unsure)
+                                                    int self, int m, unsigned unsure, bool check)
 {
     auto ord = [&](int k) { return M->o[k + 1][t]; };
     Settled<T, GEN> r{ Reach<T, GEN>(*S), m, 0, 0, 0 };
@@ -236,9 +236,10 @@ __device__ __noinline__ Settled<T, GEN> settle_ring(StarMem<T, SMALL> *M, int t,
         const typename Prec<T>::T2 a = M->q[ka][t], b = M->q[kb][t], c = M->q[kc][t];
         T o, bnd;
         turn<T>(a, b, c, err1<T>(a), err1<T>(b), err1<T>(c), o, bnd);
+        if (o > bnd && !check) continue;   // (a neighbour of one that left)
         const int e = star_recheck<GEN, false>(P, S, p, star_slot(*M, t, *S, self, ka), star_slot(*M, t, *S, self, kb),
                                                star_slot(*M, t, *S, self, kc));
-        if (o > bnd) {   // (check mode, and neighbours of one that left)
+        if (o > bnd) {
             r.mism += e < 0;
             continue;
         }
@@ -596,7 +597,7 @@ struct Star {
         // turns of the ring the filter left open: in float64
         if (CHECK) unsure = m == 32 ? ~0u : (1u << m) - 1u;
         if (R.good && unsure) {
-            const Settled<T, GEN> r = settle_ring<T, GEN, SMALL>(&M, t, &S, IDX ? A.pos : A.spos, p, self, m, unsure);
+            const Settled<T, GEN> r = settle_ring<T, GEN, SMALL>(&M, t, &S, IDX ? A.pos : A.spos, p, self, m, unsure, CHECK);
             R = r.R;
             m = r.m;
             u32 += r.u32;
