@@ -325,10 +325,10 @@ struct Star {
             // The offsets from the own slot must fit 16 bits as gather() takes them: the nearest way
             // round the set's slots if the warp wraps, as it does where this window crosses the
             // box's edge, else the plain difference (over half of the set where most points lie in
-            // a few rows).  (The nearest way in every gather: 4M uniform points 2.12 -> 2.17 ms; the
-            // edge looked at first: 1M lattice sites 308 -> 314 us.)
+            // a few rows).  (The nearest way in every gather instead: 4M uniform points 2.12 -> 2.17 ms.
+            // Branches between the conditions: 1M lattice sites 290 -> 293 us.)
             const int d = abs(s - self);
-            if (d + c > 32767 && (min(d, S.n - d) + c > 32767 || (ocy + y0 >= 0 && ocy + y1 < S.ysize))) {
+            if ((d + c > 32767) & ((min(d, S.n - d) + c > 32767) | ((ocy + y0 >= 0) & (ocy + y1 < S.ysize)))) {
                 nseg = STAR_SEGS + 1;
                 return;
             }
