@@ -52,7 +52,7 @@ BUILD_BYTES_PER_POINT = 16 + 4 + 4 + 24 + 4
 # dram__bytes_read.sum + dram__bytes_write.sum of the three launches / points) on a 1,048,576-point capture of the same
 # kernel (the --profile build case below); traffic scales with the number of points at fixed
 # density, so the 4M launch is reported as this figure times its points.
-BUILD_DRAM_BYTES_PER_POINT_NCU = 164.3
+BUILD_DRAM_BYTES_PER_POINT_NCU = 136.4
 FALLBACK_HBM_GBS = 6650.0
 
 
@@ -684,8 +684,8 @@ def run_profile_case(args):
     """A fixed, small sequence of library calls for Nsight Compute captures.  `--reps` global
     triangulations of n seeded uniform points at unit density (build, repair), or in a
     general 60-degree box at unit density (hex); with `repair`, one test-and-repair after a
-    sigma = 0.02 displacement.  Launch order per triangulation: 6 binning kernels, k_build,
-    k_build_warp.  `md`: the 256-set ensemble, one build, then `--reps` MD steps.  `mixture`:
+    sigma = 0.02 displacement.  Launch order per triangulation: 6 binning kernels, k_star twice,
+    k_wrap, k_build_warp, k_call_end.  `md`: the 256-set ensemble, one build, then `--reps` MD steps.  `mixture`:
     the 1M-point 64-cluster mixture at its tuned settings.  Prints the counters of the calls."""
     import math
 

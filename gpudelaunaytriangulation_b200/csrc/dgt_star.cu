@@ -18,7 +18,7 @@
 //      pass over the cells the circles reach, with the candidates that lie in some circle.
 // What bounds it: instruction issue (67% of the issue slots at 20 warps per SM, 22 of 32 lanes
 // active; the incremental kernel has 53% and 10 lanes, and several times the instructions).  4M
-// uniform points: 5.79 ms in the incremental kernel, 1.28 + 0.49 ms in these two launches; 1M
+// uniform points: 5.79 ms in the incremental kernel, 1.26 + 0.50 ms in these two launches; 1M
 // lattice sites 0.56 -> 0.23 ms; 1M points with float64 predicates 2.75 -> 0.67 + 0.26 ms.
 //
 // Every decision is certain or the point is handed on: a turn the filter cannot decide is
@@ -216,7 +216,7 @@ struct Reach {
 // interior, as in the pass over the stack, and leaves the ring; its neighbours' turns are looked at
 // again.  The ring's new length and reach (good: false too if a turn is not decided).
 // Near-cocircular lattices need it, half of whose diagonals stay on the stack (handing such points on
-// instead: 62,500 squares with a jitter of 1e-6 354 us, 111 in the incremental kernels, 119 so); out of
+// instead: 62,500 squares with a jitter of 1e-6 354 us, 111 in the incremental kernels, 118 so); out of
 // line, since it is rare elsewhere.
 template <typename T, bool GEN> struct Settled {
     Reach<T, GEN> R;
