@@ -65,11 +65,14 @@ constexpr int SPILL_EDGES_PER_SM = 64;
 // points per resident warp)
 constexpr int WARP_ITEMS_PER_SM = 16;
 // WRAP_BUILD_MAX's counterpart for the lists of a repair's rounds, whose length the kernels read on the
-// device (one pass
-// up to STAR_ONCE_MAX points; rebuild-only repairs of 100,000 / 250,000 jittered squares whose
-// lists hold some 35,000 points: 238 / 215 us with a warp per point up to 40,000, 166 / 190 us so).
+// device (one pass up to STAR_ONCE_MAX points).  After flips a list holds what they could not settle, and
+// its neighbours: irregular points, which a warp each takes up to a longer list (1.8M uniform points at
+// sigma 0.026, lists of some 30,000, at 20,000 / 40,000: 895 / 857 us).
+// Rebuild-only lists hold every flagged point (100,000 / 250,000 jittered squares, lists of some
+// 35,000: 166 / 190 us at 20,000, 238 / 215 us at 40,000).
 // Sets of up to WRAP_SHORT_MAX points leave the first stage out: a launch of it that finds a short
 // list costs 3 us a round.
+constexpr int WRAP_FLIP_MAX = 40000;
 constexpr int WRAP_REPAIR_MAX = 20000;
 constexpr int WRAP_SHORT_MAX = 40000;
 constexpr int MAX_DEFER_CHUNKS = 8;   // slot chunks of an overlapped global build (dgt_set_deferred_overlap)
@@ -501,8 +504,8 @@ bool hull_kernels(const dgt_context *c, int shape)
 
 // The rings of `a`'s points.  Large sets of points: the first stage with a thread per point
 // (k_star; up to STAR_ONCE_MAX points one pass of it), then with a warp per point (k_wrap) what that
-// could not finish; up to WRAP_BUILD_MAX points (repair: lists of WRAP_REPAIR_MAX): k_wrap alone,
-// whose latency is far shorter.  What is left goes
+// could not finish; up to WRAP_BUILD_MAX points (repair: lists of WRAP_REPAIR_MAX, after
+// flips WRAP_FLIP_MAX): k_wrap alone, whose latency is far shorter.  What is left goes
 // to the incremental warp kernel (exactly cocircular candidates, circles past half the box, sets
 // of a few cells).  Work budgets too small for the first stage's scans, the kernel shapes with a
 // group of lanes per point and narrow boxes leave every point to the incremental kernels instead; the kernel
@@ -517,7 +520,7 @@ cudaError_t run_rings(dgt_context *c, const RingArgs &a, cudaStream_t s, PhaseTi
     c->launches += any + 1;
     if (hull_kernels(c, shape)) {
         const bool short_lists = a.repair && a.n_items <= WRAP_SHORT_MAX;   // (k_wrap takes them whole)
-        b.wrap_items = short_lists ? a.n_items : WRAP_REPAIR_MAX;
+        b.wrap_items = short_lists ? a.n_items : (c->flip ? WRAP_FLIP_MAX : WRAP_REPAIR_MAX);
         b.star_once = STAR_ONCE_MAX;
         // (by the size of the whole build, of which `a` may be a piece: the pieces run side by side)
         b.wrap_mode = a.repair ? WRAP_REPAIR : (c->n <= WRAP_BUILD_MAX ? WRAP_OWN : WRAP_HANDED);
